@@ -202,3 +202,77 @@ def tolerance(case):
     if case["kind"] in ("block", "attention"):
         return {"rel": 1.5e-3, "max": 8e-3} if half else {"rel": 1.2e-2, "max": 6e-2}
     return {"rel": 5e-3, "max": 5e-2} if half else {"rel": 3e-2, "max": 0.25}
+
+
+# ---------------------------------------------------------------------------------------------------- 64-bit result
+def _exact_layernorm(x, gamma, beta, eps):
+    mean = x.mean(-1, keepdim=True)
+    var = ((x - mean) ** 2).mean(-1, keepdim=True)
+    return (x - mean) / torch.sqrt(var + eps) * gamma + beta
+
+
+def _exact_attention(qkv, heads, valid):
+    """softmax(Q K^T / 8) V over the valid keys, one sequence at a time (the scores of a whole batch need not fit)."""
+    B, S, W = qkv.shape
+    H = W // 3
+    out = torch.empty((B, S, H), dtype=qkv.dtype, device=qkv.device)
+    for b in range(B):
+        n = int(valid[b].sum())
+        q, k, v = (qkv[b, :, i * H:(i + 1) * H].reshape(S, heads, 64).transpose(0, 1) for i in range(3))
+        p = torch.softmax(q @ k[:, :n].transpose(1, 2) * 0.125, dim=-1)
+        out[b] = (p @ v[:, :n]).transpose(0, 1).reshape(S, H)
+    return out
+
+
+def exact(case, seed):
+    """`run`'s outputs in 64-bit floating point: the same inputs, matrix weights rounded to the compute type (the type
+    they are given to the path in), nothing else rounded."""
+    dev = torch.device("cuda")
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(seed)
+    B, S, kind = case["B"], case["S"], case["kind"]
+    dt = DTYPES[case["dtype"]]
+    lengths = np.random.default_rng(seed).integers(case["lo"], S + 1, B)
+    valid = torch.arange(S, device=dev)[None, :] < torch.from_numpy(lengths).to(dev)[:, None]
+    if kind == "attention":
+        heads = case["heads"]
+        return _exact_attention(torch.randn((B, S, 3 * heads * 64), device=dev, generator=gen).to(dt).double(), heads, valid)
+    cfg = CFGS[case["cfg"]]
+    if kind == "block":
+        cfg = EncoderConfig(1, cfg.hidden, cfg.heads, cfg.ffn, with_ffn=False)
+    weights = _Weights(cfg, gen, dev).weights
+    H, eps = cfg.hidden, cfg.ln_eps
+
+    def full(a):
+        return torch.from_numpy(a).to(dev).double()
+
+    def half(a):
+        return torch.from_numpy(a).to(dev).to(dt).double()
+
+    if kind == "reader":
+        ids = torch.randint(0, VOCAB, (B, S), device=dev, generator=gen, dtype=torch.int32)
+        segments = torch.arange(S, device=dev)[None, :] >= torch.from_numpy(lengths // 4).to(dev)[:, None]
+        word, typ, pos = ((torch.randn((rows, H), device=dev, generator=gen) * 0.02).to(dt).double()
+                          for rows in (VOCAB, 2, MAX_POS))
+        gamma = 1.0 + 0.1 * torch.randn(H, device=dev, generator=gen)
+        beta = 0.1 * torch.randn(H, device=dev, generator=gen)
+        w_qa = 0.02 * torch.randn((H, 2), device=dev, generator=gen)
+        b_qa = 0.02 * torch.randn(2, device=dev, generator=gen)
+        w_pool = 0.02 * torch.randn((H, H), device=dev, generator=gen)
+        b_pool = 0.02 * torch.randn(H, device=dev, generator=gen)
+        x = _exact_layernorm(word[ids.long()] + typ[segments.long()] + pos[:S], gamma.double(), beta.double(), eps)
+    else:
+        x = torch.randn((B, S, H), device=dev, generator=gen).double()
+    for lw in weights:
+        qkv = torch.cat([x @ half(w) + full(b) for w, b in ((lw.wq, lw.bq), (lw.wk, lw.bk), (lw.wv, lw.bv))], -1)
+        x = _exact_layernorm(_exact_attention(qkv, cfg.heads, valid) @ half(lw.wo) + full(lw.bo) + x, full(lw.ln1_g),
+                             full(lw.ln1_b), eps)
+        if cfg.with_ffn:
+            f = x @ half(lw.w1) + full(lw.b1)
+            f = 0.5 * f * (1.0 + torch.erf(f * math.sqrt(0.5)))
+            x = _exact_layernorm(f @ half(lw.w2) + full(lw.b2) + x, full(lw.ln2_g), full(lw.ln2_b), eps)
+    if kind != "reader":
+        return x
+    logits = (x.reshape(-1, H) @ w_qa.double() + b_qa.double()).T.contiguous()
+    pooled = torch.tanh(x[:, 0] @ w_pool.to(dt).double() + b_pool.double())
+    return {"hidden": x, "logits": logits, "pooled": pooled}
