@@ -78,6 +78,37 @@ def test_linear_epilogues(cuda_device, dt, epi):
 
 
 @pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("M,N,K", [
+    (1, 8, 64), (41, 768, 768), (65, 776, 320), (128, 2304, 768),      # 64 x 32 tiles
+    (128, 3072, 832), (200, 2312, 64),                                  # 64 x 64
+    (300, 3080, 128),                                                   # 128 x 64
+    (520, 3000, 192),                                                   # 128 x 128 (pair tiles with a residual)
+    (41, 768, 776),                                                     # K not in whole k-blocks: one block per stage
+])
+def test_linear_one_wave_tiles(cuda_device, dt, M, N, K):
+    """The tiles of launches that fit one wave: ragged rows, columns and last stages, strided operands, every epilogue,
+    against fp32 and bit for bit against 128 x 256 tiles with one k-block per stage (the same order of summation)."""
+    rng = np.random.default_rng(M + 5 * N + K)
+    t = lambda a: torch.from_numpy(a.astype(np.float32)).to(cuda_device)   # noqa: E731
+    x = t(rng.normal(0, 1, (M, K + 8))).to(DT[dt])[:, :K]
+    w = t(rng.normal(0, 0.05, (N, K + 24))).to(DT[dt])[:, :K]
+    r = t(rng.normal(0, 1, (M, N + 16))).to(DT[dt])[:, :N]
+    b = t(rng.normal(0, 0.5, (N,)))
+    # fp32 sums of K products of size 0.05: rounding 2^-24 per addition of a running sum below 0.2 sqrt(K), half-precision
+    # operands exact; GELU and tanh as evaluated here are within 3e-5 and 2^-11 of the exact ones
+    want = x.double() @ w.double().T + b.double()
+    for epi, ref, tol in [(ops.EPI_BIAS, want, 1e-4), (ops.EPI_BIAS_RESIDUAL, want + r.double(), 1e-4),
+                          (ops.EPI_BIAS_GELU, torch.nn.functional.gelu(want), 1e-2), (ops.EPI_BIAS_TANH, torch.tanh(want), 1e-3)]:
+        res = r if epi == ops.EPI_BIAS_RESIDUAL else None
+        y = ops.linear(x, w, b, residual=res, epilogue=epi, out_dtype=torch.float32)
+        assert (y.double() - ref).abs().max().item() < tol
+        big = torch.full((M, N + 8), 7.0, dtype=DT[dt], device=cuda_device)
+        ops.linear(x, w, b, residual=res, epilogue=epi, out=big[:, :N])
+        assert bool((big[:, N:] == 7.0).all())
+        assert torch.equal(big[:, :N], ops.linear(x, w, b, residual=res, epilogue=epi, block_n=-256))
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
 @pytest.mark.parametrize("M,N,K,bn", [(512, 768, 768, 0), (300, 1024, 256, 192), (130, 96, 64, -64), (1000, 3072, 768, 256)])
 def test_linear_layernorm_folding(cuda_device, dt, M, N, K, bn):
     """out_stats, folded input LayerNorm and folded residual LayerNorm against the unfused oracle."""

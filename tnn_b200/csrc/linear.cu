@@ -1,37 +1,52 @@
 // Projection / FFN GEMM with fused epilogue for sm_100a:  y = epilogue(x . w^T + bias (+ residual)).
 //
 // Persistent, warp-specialised CTA (one per SM):
-//   warp 0      : TMA producer   — x tile [128 x 64] and w tile [BN x 64] per k-block into a STAGES-deep ring of
-//                                   128-byte-swizzled shared memory; completion on the stage's `full` mbarrier.
+//   warp 0      : TMA producer   — x tile [TM x 64] and w tile [BN x 64] of KSUB k-blocks into one stage of a STAGES-deep
+//                                   ring of 128-byte-swizzled shared memory; completion on the stage's `full` mbarrier.
 //   warp 1      : UMMA issuer    — owns the TMEM allocation (2 accumulators of BN fp32 columns); one elected lane
-//                                   issues 4 x tcgen05.mma (128 x BN x 16) per k-block, commits the stage's `empty`
+//                                   issues 4 x tcgen05.mma (TM x BN x 16) per k-block, commits the stage's `empty`
 //                                   barrier, and commits `acc_full` after the last k-block of a tile.
-//   warps 2..9  : epilogue       — tcgen05.ld of the accumulator (a thread owns one row: lane = row), bias / GELU /
-//                                   residual in registers, 16-byte stores.  Two warps share a 32-row quarter and
-//                                   split the columns.  While they drain accumulator b, the issuer fills b^1.
+//   warps 2..   : epilogue       — tcgen05.ld of the accumulator (a thread owns one row: lane = row), bias / GELU /
+//                                   residual in registers, TMA store.  Four warps (BN = 32), or eight, of which two share
+//                                   a quarter of the rows and split the columns.  While they drain accumulator b, the
+//                                   issuer fills b^1.
+// Used where a launch has few tiles; what bounds it there is one tile's serial chain of stages.  The hand-shake of a stage
+// (wait, fence, UMMAs, commit) takes ~270 clocks whatever it holds, measured with the loads left out and a single UMMA per
+// k-block (5.1 of the 7 us that 36 more k-blocks take on a 128 x 64 tile); the UMMAs of a k-block take 50-120.  Hence several
+// k-blocks per stage, each operand fetched by one 3-D TMA box: 3072 -> 768 at 41 rows on 64 x 32 tiles 10.2 us with one
+// k-block per stage, 7.5 / 6.7 / 6.3 with two / three / four, 150 clocks per k-block, which is what the SM's read port from
+// L2 needs for the tile's 96 rows of operands.
 // Algorithmic work per launch: 2*M*N*K flop; HBM traffic at least (M*K + N*K + M*N (+ M*N residual)) elements.
 #include "linear_common.cuh"
 
 namespace b200 {
 namespace lin {
 
-template <int BN, int STAGES, bool FOLD>
+// TM = rows of a tile (128, or 64), BN = its columns, KSUB = 64-deep k-blocks per pipeline stage.
+template <int TM, int BN, int KSUB, int STAGES, bool FOLD>
 struct Cfg {
-    static constexpr int A_BYTES = BM * BK * 2;
-    static constexpr int B_BYTES = BN * BK * 2;
+    static constexpr int EPI_WARPS = BN >= 64 ? 8 : 4;          // every epilogue warp drains at least 32 columns
+    static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+    static constexpr int COLS = BN / (EPI_WARPS / 4);           // accumulator columns drained by one epilogue warp
+    static constexpr int RPW = TM / 4;                          // rows of the tile in a warp's TMEM lanes
+    static constexpr int A_BLOCK = TM * BK * 2;                 // one k-block of the tile's rows of x
+    static constexpr int B_BLOCK = BN * BK * 2;
+    static constexpr int A_BYTES = KSUB * A_BLOCK;
+    static constexpr int B_BYTES = KSUB * B_BLOCK;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int OUT_OFFSET = STAGES * STAGE_BYTES;               // output staging strips (TMA store)
-    static constexpr int BAR_OFFSET = OUT_OFFSET + kEpiWarps * kStageBytesPerWarp;
-    static constexpr int BIAS_OFFSET = BAR_OFFSET + 256;         // per-epilogue-warp bias slice: 8 x (BN/2) floats
-    static constexpr int SMEM_BYTES = BIAS_OFFSET + kEpiWarps * vec_strips<FOLD>() * (BN / 2) * 4 + 1024;  // + slack for 1024-byte alignment
-    static constexpr int TMEM_COLS = 2 * BN;                    // 128, 256 or 512: powers of two
+    static constexpr int BAR_OFFSET = OUT_OFFSET + EPI_WARPS * kStageBytesPerWarp;
+    static constexpr int BIAS_OFFSET = BAR_OFFSET + 512;         // per-epilogue-warp bias slice: COLS floats
+    static constexpr int SMEM_BYTES = BIAS_OFFSET + EPI_WARPS * vec_strips<FOLD>() * COLS * 4 + 1024;  // + slack for 1024-byte alignment
+    static constexpr int TMEM_COLS = 2 * BN;                    // 64, 128, 256 or 512: powers of two
+    static_assert((2 * STAGES + 4) * 8 + 8 <= 512, "barriers");
 };
 
-template <int BN, int STAGES, bool FOLD>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int TM, int BN, int KSUB, int STAGES, bool FOLD>
+__global__ void __launch_bounds__(Cfg<TM, BN, KSUB, STAGES, FOLD>::THREADS, 1)
 linear_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
               const __grid_constant__ CUtensorMap tm_y, const LinearParams p) {
-    using C = Cfg<BN, STAGES, FOLD>;
+    using C = Cfg<TM, BN, KSUB, STAGES, FOLD>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::BAR_OFFSET);
@@ -51,7 +66,7 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], kEpiWarps);
+            mbar_init(&acc_empty[b], C::EPI_WARPS);
         }
         *abort_flag = 0;
         mbar_fence_init();
@@ -67,25 +82,38 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        // The weights on their way from HBM into L2 while the previous kernel of the stream drains, as in the pair kernel:
+        // a prefetch reads nothing into this kernel, so it needs no order against an earlier kernel that writes them.
+        const int k_boxes = (p.num_k_blocks + KSUB - 1) / KSUB;
+        for (int b = blockIdx.x; b < k_boxes * p.num_n_tiles; b += gridDim.x) {
+            if (KSUB == 1) tma_prefetch_l2_2d(&tm_w, (b % k_boxes) * BK, (b / k_boxes) * BN);
+            else tma_prefetch_l2_3d(&tm_w, 0, (b / k_boxes) * BN, (b % k_boxes) * KSUB);
+        }
+    }
     pdl_wait();   // inputs come from earlier kernels; the output may still be read by one
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         if (elect_one()) {
-            uint32_t it = 0;
+            uint32_t st = 0, ph = 0;
             bool ok = true;
             for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
                 const int m_blk = tile / p.num_n_tiles;
                 const int n_blk = tile % p.num_n_tiles;
-                for (int kb = 0; kb < p.num_k_blocks; ++kb, ++it) {
-                    const uint32_t s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
-                    if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag)) { ok = false; break; }
-                    uint8_t* a = smem + s * C::STAGE_BYTES;
+                for (int kb = 0; kb < p.num_k_blocks; kb += KSUB) {
+                    if (!mbar_wait(&empty[st], ph ^ 1u, abort_flag)) { ok = false; break; }
+                    uint8_t* a = smem + st * C::STAGE_BYTES;
                     uint8_t* b = a + C::A_BYTES;
-                    mbar_expect_tx(&full[s], C::STAGE_BYTES);
-                    tma_load_2d(a, &tm_x, &full[s], kb * BK, m_blk * BM);
-                    tma_load_2d(b, &tm_w, &full[s], kb * BK, n_blk * BN);
+                    mbar_expect_tx(&full[st], C::STAGE_BYTES);
+                    if (KSUB == 1) {
+                        tma_load_2d(a, &tm_x, &full[st], kb * BK, m_blk * TM);
+                        tma_load_2d(b, &tm_w, &full[st], kb * BK, n_blk * BN);
+                    } else {   // maps with K split into blocks of 64: (inside the block, row, block)
+                        tma_load_3d(a, &tm_x, &full[st], 0, m_blk * TM, kb);
+                        tma_load_3d(b, &tm_w, &full[st], 0, n_blk * BN, kb);
+                    }
+                    if (++st == STAGES) { st = 0; ph ^= 1u; }
                 }
             }
             if (!ok) {
@@ -97,28 +125,33 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
     } else if (warp == 1) {
         // ------------------------------------------------------------ UMMA issuer
         if (elect_one()) {
-            uint32_t it = 0, tcount = 0;
+            uint32_t st = 0, ph = 0, tcount = 0;
             bool ok = true;
+            const uint64_t a_desc0 = make_smem_desc_sw128(smem_u32(smem));
+            const uint64_t b_desc0 = make_smem_desc_sw128(smem_u32(smem + C::A_BYTES));
             for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x, ++tcount) {
                 const uint32_t buf = tcount & 1u;
                 const uint32_t aph = (tcount >> 1) & 1u;
                 if (!mbar_wait(&acc_empty[buf], aph ^ 1u, abort_flag)) { ok = false; break; }
                 tcgen05_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int kb = 0; kb < p.num_k_blocks; ++kb, ++it) {
-                    const uint32_t s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
-                    if (!mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
+                for (int kb = 0; kb < p.num_k_blocks; kb += KSUB) {
+                    if (!mbar_wait(&full[st], ph, abort_flag)) { ok = false; break; }
                     tcgen05_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + s * C::STAGE_BYTES);
-                    const uint64_t a_desc = make_smem_desc_sw128(a_addr);
-                    const uint64_t b_desc = make_smem_desc_sw128(a_addr + C::A_BYTES);
+                    const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(st * (C::STAGE_BYTES >> 4));
+                    const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(st * (C::STAGE_BYTES >> 4));
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) {
-                        // 16 elements along K = 32 bytes inside the 128-byte swizzled row: +2 in (address >> 4) units
-                        umma_f16_ss(d_tmem, a_desc + 2u * k, b_desc + 2u * k, p.idesc, (kb | k) != 0 ? 1u : 0u);
+                    for (int sub = 0; sub < KSUB; ++sub) {
+#pragma unroll
+                        for (int k = 0; k < BK / 16; ++k) {
+                            // 16 elements along K = 32 bytes inside the 128-byte swizzled row: +2 in (address >> 4) units
+                            umma_f16_ss(d_tmem, a_desc + static_cast<uint64_t>(sub * (C::A_BLOCK >> 4) + 2 * k),
+                                        b_desc + static_cast<uint64_t>(sub * (C::B_BLOCK >> 4) + 2 * k), p.idesc,
+                                        (kb | sub | k) != 0 ? 1u : 0u);
+                        }
                     }
-                    umma_commit(&empty[s]);
+                    umma_commit(&empty[st]);
+                    if (++st == STAGES) { st = 0; ph ^= 1u; }
                 }
                 if (ok) umma_commit(&acc_full[buf]);
             }
@@ -128,11 +161,11 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
         // ------------------------------------------------------------ epilogue
         const int ew = warp - 2;
         const int quarter = warp & 3;  // TMEM lanes 32*quarter .. 32*quarter+31 are the ones this warp may read
-        const int half = ew >> 2;      // which half of the BN columns
-        constexpr int COLS = BN / 2;
+        const int half = ew >> 2;      // which COLS-wide part of the BN columns
+        constexpr int COLS = C::COLS;
         constexpr int CHUNKS = COLS / 32;
         float* vec_w = reinterpret_cast<float*>(smem + C::BIAS_OFFSET) + ew * vec_strips<FOLD>() * COLS;  // private to this warp
-        WarpEpilogue<CHUNKS, false, FOLD> epi{p, &tm_y, nullptr, smem + C::OUT_OFFSET + ew * kStageBytesPerWarp, nullptr,
+        WarpEpilogue<CHUNKS, false, FOLD, C::RPW> epi{p, &tm_y, nullptr, smem + C::OUT_OFFSET + ew * kStageBytesPerWarp, nullptr,
                                         abort_flag, lane, 0u};
         uint32_t tcount = 0;
         bool ok = true;
@@ -142,7 +175,7 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
             const uint32_t buf = tcount & 1u;
             const uint32_t aph = (tcount >> 1) & 1u;
             // Stage this tile's bias slice while the accumulator is still being produced.
-            const long long row = static_cast<long long>(m_blk) * BM + quarter * 32 + lane;
+            const long long row = static_cast<long long>(m_blk) * TM + quarter * C::RPW + lane;
             epi.begin_tile(n_blk * BN + half * COLS, static_cast<int>(row) - lane);
             stage_vectors<FOLD>(p, vec_w, n_blk * BN + half * COLS, COLS, lane);
             if (!mbar_wait(&acc_full[buf], aph, abort_flag)) { ok = false; break; }
@@ -155,7 +188,8 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[buf]);
         }
-        if (lane == 0) tma_store_wait_all<0>();   // this warp's tile stores have left shared memory and landed
+        // this warp's tile stores have read their strips; the writes themselves are complete when the grid is
+        if (lane == 0) tma_store_wait_read<0>();
         __syncwarp();
     }
 
@@ -185,22 +219,34 @@ int device_sm_count() {
     return v;
 }
 
-template <int BN, int STAGES, bool FOLD>
+template <int TM, int BN, int KSUB, int STAGES, bool FOLD>
 int launch_linear_t(const B200LinearDesc& d, cudaStream_t stream, int sm_count) {
-    using C = Cfg<BN, STAGES, FOLD>;
-    const uint64_t xd[2] = {static_cast<uint64_t>(d.K), static_cast<uint64_t>(d.M)};
-    const uint64_t xs[1] = {static_cast<uint64_t>(d.ldx) * 2};
-    const uint32_t xb[2] = {BK, BM};
-    const uint64_t wd[2] = {static_cast<uint64_t>(d.K), static_cast<uint64_t>(d.N)};
-    const uint64_t ws[1] = {static_cast<uint64_t>(d.ldw) * 2};
-    const uint32_t wb[2] = {BK, BN};
+    using C = Cfg<TM, BN, KSUB, STAGES, FOLD>;
     CUtensorMap tx, tw, ty;
-    if (!get_tensor_map(&tx, d.x, 2, xd, xs, xb) || !get_tensor_map(&tw, d.w_nk, 2, wd, ws, wb)) return B200_ERR_DRIVER;
+    if (KSUB == 1) {
+        const uint64_t xd[2] = {static_cast<uint64_t>(d.K), static_cast<uint64_t>(d.M)};
+        const uint64_t xs[1] = {static_cast<uint64_t>(d.ldx) * 2};
+        const uint32_t xb[2] = {BK, TM};
+        const uint64_t wd[2] = {static_cast<uint64_t>(d.K), static_cast<uint64_t>(d.N)};
+        const uint64_t ws[1] = {static_cast<uint64_t>(d.ldw) * 2};
+        const uint32_t wb[2] = {BK, BN};
+        if (!get_tensor_map(&tx, d.x, 2, xd, xs, xb) || !get_tensor_map(&tw, d.w_nk, 2, wd, ws, wb)) return B200_ERR_DRIVER;
+    } else {
+        // K as (K / 64) blocks of 64 (the caller has checked that K is a multiple of 64): a box covers KSUB k-blocks, which
+        // land one behind the other, each in the layout the UMMA descriptors expect.  Blocks beyond K read as zeros.
+        const uint64_t xd[3] = {BK, static_cast<uint64_t>(d.M), static_cast<uint64_t>(d.K / BK)};
+        const uint64_t xs[2] = {static_cast<uint64_t>(d.ldx) * 2, BK * 2};
+        const uint32_t xb[3] = {BK, TM, KSUB};
+        const uint64_t wd[3] = {BK, static_cast<uint64_t>(d.N), static_cast<uint64_t>(d.K / BK)};
+        const uint64_t ws[2] = {static_cast<uint64_t>(d.ldw) * 2, BK * 2};
+        const uint32_t wb[3] = {BK, BN, KSUB};
+        if (!get_tensor_map(&tx, d.x, 3, xd, xs, xb) || !get_tensor_map(&tw, d.w_nk, 3, wd, ws, wb)) return B200_ERR_DRIVER;
+    }
     ty = tx;   // placeholder when the output is fp32 (stored directly, map unused)
     if (d.out_dtype != B200_F32) {
         const uint64_t yd[2] = {static_cast<uint64_t>(d.N), static_cast<uint64_t>(d.M)};
         const uint64_t ys[1] = {static_cast<uint64_t>(d.ldy) * 2};
-        const uint32_t yb[2] = {32, 32};
+        const uint32_t yb[2] = {32, C::RPW};
         if (!get_tensor_map(&ty, d.y, 2, yd, ys, yb, 64)) return B200_ERR_DRIVER;
     }
 
@@ -217,9 +263,9 @@ int launch_linear_t(const B200LinearDesc& d, cudaStream_t stream, int sm_count) 
     p.out_dtype = d.out_dtype;
     p.epilogue = d.epilogue;
     p.num_n_tiles = (p.N + BN - 1) / BN;
-    p.num_tiles = ((p.M + BM - 1) / BM) * p.num_n_tiles;
+    p.num_tiles = ((p.M + TM - 1) / TM) * p.num_n_tiles;
     p.num_k_blocks = (p.K + BK - 1) / BK;
-    p.idesc = make_idesc_f16(BM, BN, d.dtype == B200_BF16 ? 1 : 0, 0, 0);
+    p.idesc = make_idesc_f16(TM, BN, d.dtype == B200_BF16 ? 1 : 0, 0, 0);
     p.status = device_status_ptr();
     p.out_stats = d.out_stats;
     p.ln_in_stats = d.ln_in_stats;
@@ -236,20 +282,22 @@ int launch_linear_t(const B200LinearDesc& d, cudaStream_t stream, int sm_count) 
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_once.ensure(dev, []() {
-            return cudaFuncSetAttribute(linear_kernel<BN, STAGES, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            return cudaFuncSetAttribute(linear_kernel<TM, BN, KSUB, STAGES, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         C::SMEM_BYTES) == cudaSuccess;
         }))
         return B200_ERR_LAUNCH;
     const int grid = p.num_tiles < sm_count ? p.num_tiles : sm_count;
-    launch_kernel(linear_kernel<BN, STAGES, FOLD>, dim3(grid), dim3(kThreads), C::SMEM_BYTES, stream, tx, tw, ty, p);
+    launch_kernel(linear_kernel<TM, BN, KSUB, STAGES, FOLD>, dim3(grid), dim3(C::THREADS), C::SMEM_BYTES, stream, tx, tw, ty, p);
     count_launch();
     return check_launch();
 }
 
-template <int BN, int STAGES>
+// KSUB / KSTAGES: the multi-block pipeline, for a K of whole 64-deep blocks (its maps split K into such blocks).
+template <int BN, int STAGES, int KSUB, int KSTAGES>
 int launch_linear(const B200LinearDesc& d, cudaStream_t stream, int sm_count) {
-    if (wants_fold(d)) return launch_linear_t<BN, STAGES - 1, true>(d, stream, sm_count);
-    return launch_linear_t<BN, STAGES, false>(d, stream, sm_count);
+    if (wants_fold(d)) return launch_linear_t<128, BN, 1, STAGES - 1, true>(d, stream, sm_count);
+    if (KSUB > 1 && d.K % BK == 0) return launch_linear_t<128, BN, KSUB, KSTAGES, false>(d, stream, sm_count);
+    return launch_linear_t<128, BN, 1, STAGES, false>(d, stream, sm_count);
 }
 
 // Tile choice.  Estimated time ~ waves * (columns per tile * cost per column + fixed per-tile cost), in units of
@@ -262,8 +310,26 @@ int launch_linear(const B200LinearDesc& d, cudaStream_t stream, int sm_count) {
 struct TileChoice {
     bool pair;
     int bn;
+    int tm = 128;   // rows of a single-CTA tile
 };
-TileChoice choose_tile(int64_t M, int64_t N, int sm_count) {
+TileChoice choose_tile(const B200LinearDesc& d, int sm_count) {
+    const int64_t M = d.M, N = d.N;
+    // Few rows: a launch is bound by its latencies (hand-over, first loads, the serial chain of k-blocks of one tile, drain),
+    // so the smallest tile that still fits one wave is the fastest: the more SMs fetch operands at once, the shorter each
+    // one's chain.  12 launches in turn on weights of their own, us per launch, before (128 x 64 tiles, one k-block per
+    // stage) -> on the tile below:  M = 41: 768 -> 768 4.8 -> 3.5, 768 -> 2304 4.6 -> 3.4, 768 -> 3072 4.9 -> 4.0,
+    // 3072 -> 768 11.1 -> 6.3;  M = 256: 5.1 -> 3.7, 4.9 -> 4.2, 5.4 -> 5.1, 11.7 -> 6.8;  M = 1024: 768 -> 768 5.4 -> 5.1,
+    // 3072 -> 768 12.7 -> 10.7 (128 x 64).  One tile more than SMs and the next wider one is ahead: 768 -> 3072 at 128 rows
+    // 4.9 on 192 tiles of 64 x 32, 4.5 on 96 of 64 x 64.  All tiles add a row's products up in the same order, so the choice
+    // changes no bit of the result.
+    if (!wants_fold(d) && d.K % BK == 0) {
+        const struct { int tm, bn; } small[3] = {{64, 32}, {64, 64}, {128, 64}};
+        for (const auto& t : small)
+            if (((M + t.tm - 1) / t.tm) * ((N + t.bn - 1) / t.bn) <= sm_count) return {false, t.bn, t.tm};
+        // 128 x 128 drains two chunks per warp, and a residual of the second is not fetched ahead: 768 -> 2304 at 1024 rows
+        // 5.9 against 6.4 us on pair tiles, 768 -> 768 with a residual at 2048 rows 8.1 against 6.7.
+        if (d.epilogue != B200_EPI_BIAS_RESIDUAL && ((M + 127) / 128) * ((N + 127) / 128) <= sm_count) return {false, 128};
+    }
     TileChoice best = {false, 128};
     double best_t = 1e300;
     if (M > 128) {
@@ -277,7 +343,7 @@ TileChoice choose_tile(int64_t M, int64_t N, int sm_count) {
             const double t = static_cast<double>(waves) * (bns[i] * cost[i] + 16.0);
             if (t < best_t) {
                 best_t = t;
-                best = {true, bns[i]};
+                best = {true, bns[i], 128};
             }
         }
     }
@@ -289,7 +355,7 @@ TileChoice choose_tile(int64_t M, int64_t N, int sm_count) {
         const double t = static_cast<double>(waves) * (bns1[i] * cost1[i] + 16.0);
         if (t < best_t) {
             best_t = t;
-            best = {false, bns1[i]};
+            best = {false, bns1[i], 128};
         }
     }
     return best;
@@ -328,11 +394,11 @@ extern "C" int b200_linear_fwd(const B200LinearDesc* d, b200_stream_t stream_) {
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     TileChoice tc;
     if (d->block_n == 0) {
-        tc = choose_tile(d->M, d->N, sms);
+        tc = choose_tile(*d, sms);
     } else if (d->block_n > 0) {
-        tc = {d->M > 128, d->block_n};
+        tc = {d->M > 128, d->block_n, 128};
     } else {
-        tc = {false, -d->block_n};
+        tc = {false, -d->block_n, 128};
     }
     if (tc.pair) {
         switch (tc.bn) {
@@ -343,10 +409,14 @@ extern "C" int b200_linear_fwd(const B200LinearDesc* d, b200_stream_t stream_) {
             default: return B200_ERR_PARAM;
         }
     }
+    if (tc.tm == 64) {
+        return tc.bn == 32 ? launch_linear_t<64, 32, 4, 4, false>(*d, stream, sms)
+                           : launch_linear_t<64, 64, 4, 3, false>(*d, stream, sms);
+    }
     switch (tc.bn) {
-        case 256: return launch_linear<256, 4>(*d, stream, sms);
-        case 128: return launch_linear<128, 6>(*d, stream, sms);
-        case 64: return launch_linear<64, 8>(*d, stream, sms);
+        case 256: return launch_linear<256, 4, 1, 4>(*d, stream, sms);
+        case 128: return launch_linear<128, 6, 2, 3>(*d, stream, sms);
+        case 64: return launch_linear<64, 8, 2, 4>(*d, stream, sms);
         default: return B200_ERR_PARAM;
     }
 }

@@ -135,7 +135,7 @@ constexpr int kStageBytesPerWarp = 32 * 64;
 template <bool RES> constexpr int strips_per_warp() { return RES ? 3 : 1; }
 template <bool FOLD> constexpr int vec_strips() { return FOLD ? 4 : 1; }   // bias|c2, c1, gamma, beta
 
-template <int CHUNKS, bool RES, bool FOLD>
+template <int CHUNKS, bool RES, bool FOLD, int RPW = 32>
 struct WarpEpilogue {
     static constexpr int NSTRIPS = RES ? 3 : 1;
     const LinearParams& p;
@@ -158,6 +158,14 @@ struct WarpEpilogue {
     // bit s of `rpar` is the phase parity of strip s's residual barrier (it flips with every residual tile received).
     uint32_t rpar = 0;
     bool res_on = true;
+    // A warp that drains a single chunk per tile reads its residual straight from global memory, but ahead of the wait for
+    // the accumulator: the loads (an L2 or HBM round trip) overlap the tile's mainloop.
+    static constexpr bool kEarlyResidual = !RES && CHUNKS == 1;
+    uint4 early[kEarlyResidual ? 4 : 1];
+
+    // RPW = rows of a tile per warp: 32 (tiles of 128 rows), or 16 (64 rows: the accumulator's rows sit in the lower half
+    // of each warp's TMEM lanes, so lanes 16 .. 31 of the warp have no row)
+    __device__ __forceinline__ bool has_row(long long row) const { return row < p.M && (RPW == 32 || lane < RPW); }
 
     __device__ __forceinline__ bool ln_in() const { return FOLD && p.ln_in_stats != nullptr; }
     __device__ __forceinline__ bool res_ln() const { return FOLD && p.res_ln_stats != nullptr; }
@@ -202,6 +210,13 @@ struct WarpEpilogue {
     // Call before waiting for the accumulator: overlaps the first residual load with the tile's mainloop.
     __device__ __forceinline__ void begin_tile(int n_first, int row0) {
         if (RES && res_on && chunk_valid(0, n_first, row0)) issue_residual(cc, n_first, row0);
+        if (kEarlyResidual && p.epilogue == B200_EPI_BIAS_RESIDUAL && has_row(static_cast<long long>(row0) + lane)) {
+            const uint16_t* rp = reinterpret_cast<const uint16_t*>(p.residual) +
+                                 (static_cast<long long>(row0) + lane) * p.ldr + n_first;
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+                if (n_first + g * 8 < p.N) early[g] = *reinterpret_cast<const uint4*>(rp + g * 8);
+        }
         if (!FOLD) return;
         const long long row = static_cast<long long>(row0) + lane;
         const bool have_pf = pf_row == row && row < p.M;
@@ -256,7 +271,7 @@ struct WarpEpilogue {
     // of the accumulator's column 0 with this warp's lane offset already applied.  Returns false if a wait ran out.
     template <int COLS>
     __device__ __forceinline__ bool run(const float* vec_w, uint32_t tacc, long long row, int n_tile0, int col_first) {
-        const bool row_ok = row < p.M;
+        const bool row_ok = has_row(row);
         const int row0 = static_cast<int>(row) - lane;
         const int n_first = n_tile0 + col_first;
         uint32_t r[32];
@@ -321,7 +336,7 @@ struct WarpEpilogue {
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
                     if (n0 + g * 8 < p.N) {
-                        const uint4 q = __ldg(reinterpret_cast<const uint4*>(rp + g * 8));
+                        const uint4 q = kEarlyResidual ? early[g] : __ldg(reinterpret_cast<const uint4*>(rp + g * 8));
                         add_residual8<COLS>(q, vec_w, c * 32 + g * 8, &v[g * 8]);
                     }
                 }

@@ -85,6 +85,11 @@ __device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* map, int32
                  ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1)
                  : "memory");
 }
+__device__ __forceinline__ void tma_prefetch_l2_3d(const CUtensorMap* map, int32_t c0, int32_t c1, int32_t c2) {
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
+}
 // 2-D tile load global -> this CTA's shared memory, completion on `bar` (complete_tx bytes).
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int32_t c0, int32_t c1) {
     asm volatile(
