@@ -268,6 +268,22 @@ def test_attention_mask_with_holes_and_no_mask(cuda_device):
     assert max_abs(_np(out), want) < 6e-3
 
 
+@pytest.mark.parametrize("S", [384, 640, 300])
+def test_attention_of_a_batch_equals_its_sequences_alone(cuda_device, S):
+    """Sequence lengths whose last query block has at most 128 rows: a CTA then walks items with and without a second
+    query tile.  Every sequence of a ragged batch (more items than CTAs) must give, bit for bit, what it gives alone, in
+    every one of several runs."""
+    B, heads = 40, 12
+    gen = torch.Generator(device=cuda_device).manual_seed(S)
+    qkv = torch.randn((B, S, 3 * heads * 64), device=cuda_device, generator=gen).half()
+    lens = torch.randint(1, S + 1, (B,), device=cuda_device, generator=gen)
+    mask = torch.where(torch.arange(S, device=cuda_device)[None] < lens[:, None], 0.0, -10000.0).contiguous()
+    kv = ops.mask_to_kv_len(mask)
+    alone = torch.cat([ops.attention(qkv[b:b + 1], heads, mask[b:b + 1], kv[b:b + 1]) for b in range(B)])
+    for _ in range(10):
+        assert torch.equal(ops.attention(qkv, heads, mask, kv), alone)
+
+
 @pytest.mark.parametrize("S,lengths", [(256, [77, 200]), (128, [5, 100]), (96, [33, 96])])
 def test_attention_padded_keys_have_exactly_zero_weight(cuda_device, S, lengths):
     """Perturbing K/V rows of padded keys must leave every output bit-identical."""

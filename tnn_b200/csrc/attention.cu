@@ -778,8 +778,12 @@ attention_pingpong_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, c
             for (int j = 0; j < n_tiles; ++j, ++u, ++t) {
                 const int st = static_cast<int>(t % PP_NST);
                 const uint32_t ph = u & 1u;
-                if (!mbar_wait(&m_full[st], (t / PP_NST) & 1u, abort_flag)) { ok = false; break; }
+                // The scores first: warpgroup 1 skips items in which it has no rows and may get here before the producer has
+                // even reached the stage's previous tile, and a parity wait would take that for the phase meant.  Once the
+                // scores are complete the producer has fetched K of this tile, hence published the masks of the tiles four
+                // and more before it, and the stage's barrier is in this tile's phase.
                 if (!mbar_wait(&s_full[wg], ph, abort_flag)) { ok = false; break; }
+                if (!mbar_wait(&m_full[st], (t / PP_NST) & 1u, abort_flag)) { ok = false; break; }
                 __syncwarp();
                 tcgen05_fence_after();
                 // The row's 128 scores move to registers in one go and the score columns are handed back at once:
