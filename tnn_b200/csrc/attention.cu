@@ -245,8 +245,11 @@ attention_pingpong_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         } else if (warp == 1 || (NWG == 2 && warp == 2 && two)) {
             // ------------------------------------------------------------ UMMA issuers (one warp per warpgroup)
             // The whole warp runs this role's control flow (all waits, all address arithmetic: warp-uniform, every
-            // descriptor an immediate offset from one built once); lane 0 alone executes the tcgen05.mma and
-            // tcgen05.commit instructions, so that each commit covers the UMMAs before it.
+            // descriptor an immediate offset from one built once); one elected lane alone executes the tcgen05.mma and
+            // tcgen05.commit instructions, so that each commit covers the UMMAs before it.  The lane is named by
+            // elect.sync, which tells the compiler that the block has a single thread: with `lane == 0` the operands went
+            // through per-lane registers, and the issuers' steps lie on every tile's critical path
+            // (16 x 2048 tokens, 16 heads: 429 -> 416 us; the role as one thread altogether: 421).
             bool ok = mbar_wait(q_full, 0, abort_flag);
             const uint32_t idesc_qk = p.idesc_qk, idesc_pv = p.idesc_pv;
             const uint64_t dq0 = make_smem_desc_sw128(smem_u32(smem + PP_OFF_Q));   // descriptor addresses: 16-byte units
@@ -254,7 +257,7 @@ attention_pingpong_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             const uint64_t dv0 = make_smem_desc_sw128(smem_u32(smem + PP_OFF_V));
             auto issue_s = [&](auto wg_c, const int st) {
                 constexpr int wg = decltype(wg_c)::value;
-                if (lane == 0) {
+                if (elect_one()) {
                     const uint64_t a_desc = dq0 + static_cast<uint64_t>(wg * (TILE_BYTES >> 4));
                     const uint64_t b_desc = dk0 + static_cast<uint64_t>(st * (TILE_BYTES >> 4));
                     const uint32_t d_tmem = tmem_base + wg * 128;
@@ -285,7 +288,7 @@ attention_pingpong_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 if (!mbar_wait(&p_full[wg], static_cast<uint32_t>(j) & 1u, abort_flag)) return false;
                 if (!mbar_wait(&v_full[st], (static_cast<uint32_t>(j) / PP_NST) & 1u, abort_flag)) return false;
                 tcgen05_fence_after();
-                if (lane == 0) {
+                if (elect_one()) {
                     const uint64_t b_desc = dv0 + static_cast<uint64_t>(st * (TILE_BYTES >> 4));
                     const uint32_t d_tmem = tmem_base + C::COL_O + wg * 64;
                     const uint32_t a_tmem = tmem_base + C::COL_P + wg * 64;
@@ -484,7 +487,7 @@ attention_pingpong_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 // warpgroups fall into, and that relation reacted to every restructuring that was measured (this form run with one
 // item per CTA is 5-8 % slower than the kernel above on items of 16 and 32 tiles; with the UMMA-issuing warps
 // specialised at compile time it is 8-16 % slower than as written here), so each form keeps the code it was tuned with.
-template <int DT, int NWG>
+template <int DT, int NWG, bool ONE>
 __global__ void __launch_bounds__(PPCfg<NWG, 2>::THREADS, PPCfg<NWG, 2>::CTAS_PER_SM)
 attention_pingpong_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                           const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
@@ -569,10 +572,13 @@ attention_pingpong_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, c
     };
     auto load_item = [&](int id) -> Item {
         Item it;
-        const int qb = id % p.n_qb;
-        const int rest = id / p.n_qb;
-        it.head = rest % p.heads;
-        it.b = rest / p.heads;
+        // Heads vary fastest, then the query blocks of a sequence: with the query blocks fastest and an even number of them,
+        // a grid of 148 dealt every second CTA nothing but last blocks, which for S = 384 (a last block of 128 queries
+        // instead of 256) left half of the CTAs with half of the work: 64 x 384 tokens, 16 heads: 110.9 us, now 101.7.
+        it.head = id % p.heads;
+        const int rest = id / p.heads;
+        const int qb = rest % p.n_qb;
+        it.b = rest / p.n_qb;
         it.q0 = qb * NWG * TQ;
         it.two = NWG == 2 && (p.S - it.q0) > TQ;
         // kv_len is written by a kernel earlier in the stream: it is read only here, behind the dependency wait.
@@ -647,12 +653,17 @@ attention_pingpong_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, c
             __syncwarp();
         } else if (warp == 1 || (NWG == 2 && warp == 2)) {
             // ------------------------------------------------------------ UMMA issuers (one warp per warpgroup)
-            // The whole warp runs this role's control flow (all waits, all address arithmetic: warp-uniform, every
-            // descriptor an immediate offset from one built once); lane 0 alone executes the tcgen05.mma and
-            // tcgen05.commit instructions, so that each commit covers the UMMAs before it.  Both warps walk every
-            // item: where an item has no second query tile, warp 2 issues nothing but still waits for the stage's
-            // loads and commits, so that every "empty" barrier gets its NWG arrivals once per use and in step.
+            // ONE: one elected lane runs the role (polls, addresses, UMMAs and commits).  Otherwise the whole warp runs its
+            // control flow (waits and address arithmetic) and lane 0 alone executes the tcgen05 instructions, so that each
+            // commit covers the UMMAs before it.  The issuers' steps lie on every tile's critical path and the single lane
+            // is the faster one, but the form also shifts the phase relation of the two softmax warpgroups, and over items
+            // of many tiles that decides (launch_pingpong draws the line).  Both warps walk every item: where an item has
+            // no second query tile, warp 2 issues nothing but still waits for the stage's loads and commits, so that every
+            // "empty" barrier gets its NWG arrivals once per use and in step.
+            // (Leaving out the 32-key chunks of a sequence's last key tile that hold no keys, here and in the softmax, was
+            // measured and is not worth its code: 16 x 512 full 39.4 -> 40.8 us, 64 x 384 of 128 .. 384 valid 93.8 -> 101.8.)
             const int wg = warp - 1;
+            if (!ONE || elect_one()) {
             const uint32_t idesc_qk = p.idesc_qk, idesc_pv = p.idesc_pv;
             const uint64_t dq0 = make_smem_desc_sw128(smem_u32(smem + PP_OFF_Q));   // descriptor addresses: 16-byte units
             const uint64_t dk0 = make_smem_desc_sw128(smem_u32(smem + PP_OFF_K));   // + stage * (TILE_BYTES >> 4)
@@ -670,7 +681,7 @@ attention_pingpong_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, c
                 if (active && u_s > 0 && !mbar_wait(&s_free[wg], (u_s - 1u) & 1u, abort_flag)) return false;
                 if (!mbar_wait(&k_full[st], (t / PP_NST) & 1u, abort_flag)) return false;
                 tcgen05_fence_after();
-                if (lane == 0) {
+                if (ONE || lane == 0) {
                     if (active) {
                         const uint64_t a_desc = dq0 + static_cast<uint64_t>((set * NWG + wg) * (TILE_BYTES >> 4));
                         const uint64_t b_desc = dk0 + static_cast<uint64_t>(st * (TILE_BYTES >> 4));
@@ -683,7 +694,7 @@ attention_pingpong_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, c
                     umma_commit(&k_empty[st]);
                     if (j == n - 1) umma_commit(&q_empty[set]);
                 }
-                __syncwarp();
+                if (!ONE) __syncwarp();
                 if (active) ++u_s;
                 return true;
             };
@@ -695,7 +706,7 @@ attention_pingpong_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, c
                 if (active && !mbar_wait(&p_full[wg], u_pv & 1u, abort_flag)) return false;
                 if (!mbar_wait(&v_full[st], (t / PP_NST) & 1u, abort_flag)) return false;
                 tcgen05_fence_after();
-                if (lane == 0) {
+                if (ONE || lane == 0) {
                     if (active) {
                         const uint64_t b_desc = dv0 + static_cast<uint64_t>(st * (TILE_BYTES >> 4));
                         const uint32_t d_tmem = tmem_base + C::COL_O + wg * 64;
@@ -711,7 +722,7 @@ attention_pingpong_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, c
                     }
                     umma_commit(&v_empty[st]);
                 }
-                __syncwarp();
+                if (!ONE) __syncwarp();
                 if (active) ++u_pv;
                 return true;
             };
@@ -724,7 +735,8 @@ attention_pingpong_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, c
                 const Item it = load_item(id);
                 n = it.n_tiles;
                 two_ = it.two;
-                ok = __all_sync(0xffffffffu, issue_s(k, t0, n, two_, 0));
+                ok = issue_s(k, t0, n, two_, 0);
+                if (!ONE) ok = __all_sync(0xffffffffu, ok);
             }
             while (ok && id < n_items) {
                 const int id_n = id + id_step;
@@ -740,13 +752,14 @@ attention_pingpong_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, c
                     if (j + 1 < n) ok = issue_s(k, t0, n, two_, j + 1);
                     else if (id_n < n_items) ok = issue_s(k + 1, t0 + static_cast<uint32_t>(n), n_n, two_n, 0);
                     if (ok) ok = issue_pv(t0, two_, j);
-                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ONE) ok = __all_sync(0xffffffffu, ok);
                 }
                 t0 += static_cast<uint32_t>(n);
                 id = id_n;
                 ++k;
                 n = n_n;
                 two_ = two_n;
+            }
             }
             __syncwarp();
         }
@@ -1227,9 +1240,13 @@ bool set_attention_attributes(int dev) {
                                  PPCfg<PP_NWG, 1>::SMEM) == cudaSuccess &&
             cudaFuncSetAttribute(attention_pingpong_kernel<B200_BF16, PP_NWG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  PPCfg<PP_NWG, 1>::SMEM) == cudaSuccess &&
-            cudaFuncSetAttribute(attention_pingpong_persistent_kernel<B200_F16, PP_NWG>,
+            cudaFuncSetAttribute(attention_pingpong_persistent_kernel<B200_F16, PP_NWG, true>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, PPCfg<PP_NWG, 2>::SMEM) == cudaSuccess &&
-            cudaFuncSetAttribute(attention_pingpong_persistent_kernel<B200_BF16, PP_NWG>,
+            cudaFuncSetAttribute(attention_pingpong_persistent_kernel<B200_BF16, PP_NWG, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, PPCfg<PP_NWG, 2>::SMEM) == cudaSuccess &&
+            cudaFuncSetAttribute(attention_pingpong_persistent_kernel<B200_F16, PP_NWG, false>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, PPCfg<PP_NWG, 2>::SMEM) == cudaSuccess &&
+            cudaFuncSetAttribute(attention_pingpong_persistent_kernel<B200_BF16, PP_NWG, false>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, PPCfg<PP_NWG, 2>::SMEM) == cudaSuccess;
         if (!ok) cudaGetLastError();
         return ok;
@@ -1253,16 +1270,17 @@ int launch_pingpong(AttnParams& p, int dtype, long long S, int heads, long long 
         const dim3 grid(static_cast<unsigned>(p.n_items < slots ? p.n_items : slots));
         const dim3 block(PPCfg<PP_NWG, 2>::THREADS);
         constexpr size_t smem = PPCfg<PP_NWG, 2>::SMEM;
-        if (with_attributes) {
-            if (dtype == B200_F16)
-                launch_kernel(attention_pingpong_persistent_kernel<B200_F16, PP_NWG>, grid, block, smem, stream, tq, tk, tv, p);
-            else
-                launch_kernel(attention_pingpong_persistent_kernel<B200_BF16, PP_NWG>, grid, block, smem, stream, tq, tk, tv, p);
-        } else if (dtype == B200_F16) {
-            attention_pingpong_persistent_kernel<B200_F16, PP_NWG><<<grid, block, smem, stream>>>(tq, tk, tv, p);
-        } else {
-            attention_pingpong_persistent_kernel<B200_BF16, PP_NWG><<<grid, block, smem, stream>>>(tq, tk, tv, p);
-        }
+        // Issuers as one lane up to six key tiles, as a whole warp beyond, us per launch with 16 or 12 heads, whole warp ->
+        // one lane: 64 x 384 101.7 -> 93.8, 16 x 512 40.0 -> 39.4, 32 x 256 21.7 -> 20.7, 8 x 640 (100 .. 640 valid) 27.9 ->
+        // 26.0;  16 x 1024 116.1 -> 120.4, of 200 .. 1024 valid 96.8 -> 98.9.
+        const bool one = S <= 6 * TK;
+        auto kernel = dtype == B200_F16
+                          ? (one ? attention_pingpong_persistent_kernel<B200_F16, PP_NWG, true>
+                                 : attention_pingpong_persistent_kernel<B200_F16, PP_NWG, false>)
+                          : (one ? attention_pingpong_persistent_kernel<B200_BF16, PP_NWG, true>
+                                 : attention_pingpong_persistent_kernel<B200_BF16, PP_NWG, false>);
+        if (with_attributes) launch_kernel(kernel, grid, block, smem, stream, tq, tk, tv, p);
+        else kernel<<<grid, block, smem, stream>>>(tq, tk, tv, p);
         return B200_OK;
     }
     const dim3 grid(static_cast<unsigned>(n_qb), static_cast<unsigned>(heads), static_cast<unsigned>(B));
