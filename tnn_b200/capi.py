@@ -138,14 +138,14 @@ def check(code, where):
         raise B200Error(code, where)
 
 
+_DTYPE_CODES = {torch.float16: F16, torch.bfloat16: BF16, torch.float32: F32}
+
+
 def dtype_code(dt):
-    if dt == torch.float16:
-        return F16
-    if dt == torch.bfloat16:
-        return BF16
-    if dt == torch.float32:
-        return F32
-    raise ValueError("unsupported dtype %s" % dt)
+    code = _DTYPE_CODES.get(dt)
+    if code is None:
+        raise ValueError("unsupported dtype %s" % dt)
+    return code
 
 
 def torch_dtype(code):
@@ -156,7 +156,13 @@ def ptr(t):
     return None if t is None else t.data_ptr()
 
 
+# The current stream's handle without the Stream object around it, where this torch offers that (1.0 -> 0.3 us a call).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_ptr():
+    if _raw_stream is not None:
+        return _raw_stream(torch.cuda.current_device())
     return torch.cuda.current_stream().cuda_stream
 
 

@@ -81,9 +81,10 @@ class Encoder:
         if mask_add is not None:
             m2 = mask_add.reshape(B, S).contiguous()
             kv_len = ops.mask_to_kv_len(m2)
+        scale = 1.0 / float(np.sqrt(cfg.head_dim))
         for L in self.layers:
             qkv = ops.linear(h, L["w_qkv"], L["b_qkv"])
-            ctx = ops.attention(qkv, cfg.heads, m2, kv_len, scale=1.0 / float(np.sqrt(cfg.head_dim)))
+            ctx = ops.attention(qkv, cfg.heads, m2, kv_len, scale=scale)
             t = ops.linear(ctx, L["w_o"], L["b_o"], residual=h, epilogue=ops.EPI_BIAS_RESIDUAL)
             a = ops.add_layernorm(t, L["ln1_g"], L["ln1_b"], cfg.ln_eps)
             if cfg.with_ffn:
@@ -162,18 +163,9 @@ class Encoder:
         if not self.cfg.with_ffn:
             raise ValueError("b200_encoder_fwd runs full encoder layers; use forward_ops for attention-only blocks")
         B, S, H = hidden.shape
-        d = capi.EncoderDesc()
-        d.hidden = hidden.data_ptr()
-        d.mask_add = capi.ptr(mask2d)
-        d.kv_len = capi.ptr(kv_len)
-        d.layers = self._layer_array()
-        d.workspace = self.workspace(B * S)
-        d.B, d.S, d.H, d.F = B, S, H, self.cfg.ffn
-        d.heads, d.num_layers = self.cfg.heads, len(self.layers)
-        d.dtype = capi.dtype_code(self.dtype)
-        d.ln_eps = float(self.cfg.ln_eps)
-        d.mask_exclude_below = -5000.0
-        d.fold_layernorm = 1 if self.fold else 0
+        d = capi.EncoderDesc(hidden.data_ptr(), capi.ptr(mask2d), capi.ptr(kv_len), self._layer_array(),
+                             self.workspace(B * S), B, S, H, self.cfg.ffn, self.cfg.heads, len(self.layers),
+                             capi.dtype_code(self.dtype), float(self.cfg.ln_eps), -5000.0, 1 if self.fold else 0)
         rc = capi.lib().b200_encoder_fwd(ctypes.byref(d), capi.stream_ptr())
         capi.check(rc, "b200_encoder_fwd")
         return hidden

@@ -18,6 +18,16 @@ def _require_cuda(*ts):
             raise ValueError("tnn_b200 operators take CUDA tensors only (there is no CPU path)")
 
 
+def _rows(t, width):
+    """`t` as rows of `width` elements: (tensor that holds them, number of rows, row stride).  A contiguous tensor, the
+    usual one, needs no view of its own: making views costs more than filling a descriptor."""
+    if t.is_contiguous():
+        return t, t.numel() // width, width
+    t2 = t.reshape(-1, width)
+    assert t2.stride(1) == 1
+    return t2, t2.shape[0], t2.stride(0)
+
+
 def pack_weight(w_kn, dtype=torch.float16, out=None):
     """fp32 `[K, N]` (TNN MatMul weight layout, y = x.W) -> `dtype` `[N, K]` on the device."""
     _require_cuda(w_kn)
@@ -69,24 +79,18 @@ def _linear_desc(x, w_nk, bias, residual, epilogue, out_dtype, out, block_n, out
                  ln_eps=1e-12):
     _require_cuda(x, w_nk, bias, residual, out)
     K = x.shape[-1]
-    x2 = x.reshape(-1, K)
-    M = x2.shape[0]
     N = w_nk.shape[0]
-    assert w_nk.shape[1] == K and x2.stride(1) == 1 and w_nk.stride(1) == 1
-    out_dtype = out_dtype or x.dtype
+    assert w_nk.shape[1] == K and w_nk.stride(1) == 1
+    x2, M, ldx = _rows(x, K)
     if out is None:
-        out = torch.empty(x.shape[:-1] + (N,), dtype=out_dtype, device=x.device)
-    y2 = out.reshape(-1, N)
-    d = capi.LinearDesc()
-    d.x, d.w_nk, d.bias, d.y = x2.data_ptr(), w_nk.data_ptr(), capi.ptr(bias), y2.data_ptr()
-    d.M, d.N, d.K = M, N, K
-    d.ldx, d.ldw, d.ldy = x2.stride(0), w_nk.stride(0), y2.stride(0)
+        out = torch.empty(x.shape[:-1] + (N,), dtype=out_dtype or x.dtype, device=x.device)
+    y2, _, ldy = _rows(out, N)
+    d = capi.LinearDesc(x2.data_ptr(), w_nk.data_ptr(), capi.ptr(bias), None, y2.data_ptr(), M, N, K, ldx,
+                        w_nk.stride(0), 0, ldy, capi.dtype_code(x.dtype), capi.dtype_code(out.dtype), epilogue, block_n)
     if residual is not None:
-        r2 = residual.reshape(-1, N)
-        assert r2.dtype == x.dtype and r2.stride(1) == 1
-        d.residual, d.ldr = r2.data_ptr(), r2.stride(0)
-    d.dtype, d.out_dtype = capi.dtype_code(x.dtype), capi.dtype_code(out.dtype)
-    d.epilogue, d.block_n = epilogue, block_n
+        assert residual.dtype == x.dtype
+        r2, _, d.ldr = _rows(residual, N)
+        d.residual = r2.data_ptr()
     # LayerNorm folding: ln_in = (stats of x, c1, c2); res_ln = (stats of residual, gamma, beta)
     d.ln_eps = float(ln_eps)
     if out_stats is not None:
@@ -130,21 +134,17 @@ def attention(qkv, heads, mask_add=None, kv_len=None, scale=None, exclude_below=
     if out is None:
         out = torch.empty((B, S, H), dtype=qkv.dtype, device=qkv.device)
     es = qkv.element_size()
-    d = capi.AttentionDesc()
-    d.q, d.k, d.v = qkv.data_ptr(), qkv.data_ptr() + H * es, qkv.data_ptr() + 2 * H * es
-    d.ldq = d.ldk = d.ldv = qkv.stride(1)
-    d.out, d.ldo = out.data_ptr(), out.stride(1)
+    q = qkv.data_ptr()
+    ld = qkv.stride(1)
+    d = capi.AttentionDesc(q, q + H * es, q + 2 * H * es, None, None, out.data_ptr(), B, S, ld, ld, ld, out.stride(1), heads,
+                           64, capi.dtype_code(qkv.dtype), 0.125 if scale is None else float(scale), float(exclude_below))
     if mask_add is not None:
-        m2 = mask_add.reshape(B, S)
+        m2 = mask_add if mask_add.is_contiguous() and mask_add.numel() == B * S else mask_add.reshape(B, S)
         assert m2.is_contiguous() and m2.dtype == torch.float32
         d.mask_add = m2.data_ptr()
     if kv_len is not None:
         assert kv_len.dtype == torch.int32 and kv_len.numel() == B
         d.kv_len = kv_len.data_ptr()
-    d.B, d.S, d.heads, d.head_dim = B, S, heads, 64
-    d.dtype = capi.dtype_code(qkv.dtype)
-    d.scale = float(scale if scale is not None else 0.125)
-    d.mask_exclude_below = float(exclude_below)
     rc = capi.lib().b200_attention_fwd(ctypes.byref(d), capi.stream_ptr())
     capi.check(rc, "b200_attention_fwd")
     return out
@@ -153,19 +153,17 @@ def attention(qkv, heads, mask_add=None, kv_len=None, scale=None, exclude_below=
 def _layernorm_desc(x, gamma, beta, eps, residual, out_dtype, out):
     _require_cuda(x, gamma, beta, residual, out)
     H = x.shape[-1]
-    x2 = x.reshape(-1, H)
-    assert x2.stride(1) == 1 and gamma.dtype == torch.float32 and beta.dtype == torch.float32
+    assert gamma.dtype == torch.float32 and beta.dtype == torch.float32
+    x2, rows, ldx = _rows(x, H)
     if out is None:
         out = torch.empty(x.shape, dtype=out_dtype or x.dtype, device=x.device)
-    y2 = out.reshape(-1, H)
-    d = capi.LayerNormDesc()
-    d.x, d.gamma, d.beta, d.y = x2.data_ptr(), gamma.data_ptr(), beta.data_ptr(), y2.data_ptr()
-    d.rows, d.H, d.ldx, d.ldy = x2.shape[0], H, x2.stride(0), y2.stride(0)
+    y2, _, ldy = _rows(out, H)
+    d = capi.LayerNormDesc(x2.data_ptr(), None, gamma.data_ptr(), beta.data_ptr(), y2.data_ptr(), rows, H, ldx, 0, ldy,
+                           capi.dtype_code(x.dtype), capi.dtype_code(out.dtype), float(eps))
     if residual is not None:
-        r2 = residual.reshape(-1, H)
-        assert r2.dtype == x.dtype
-        d.residual, d.ldr = r2.data_ptr(), r2.stride(0)
-    d.in_dtype, d.out_dtype, d.eps = capi.dtype_code(x.dtype), capi.dtype_code(out.dtype), float(eps)
+        assert residual.dtype == x.dtype
+        r2, _, d.ldr = _rows(residual, H)
+        d.residual = r2.data_ptr()
     return d, out
 
 
