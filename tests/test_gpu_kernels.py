@@ -109,6 +109,25 @@ def test_linear_one_wave_tiles(cuda_device, dt, M, N, K):
 
 
 @pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("bn", [64, 128])
+@pytest.mark.parametrize("M,N,K", [(129, 72, 64), (300, 200, 320), (257, 776, 1088), (2500, 776, 192), (300, 200, 328)])
+def test_linear_pair_tiles_with_two_k_blocks_per_stage(cuda_device, dt, bn, M, N, K):
+    """CTA-pair tiles whose stages hold two k-blocks (K of whole blocks; 328 is not): odd block counts, one and several
+    tiles per pair, strided operands, with and without a residual, bit for bit as 128 x 256 tiles give it."""
+    gen = torch.Generator(device=cuda_device).manual_seed(M + N + K)
+    x = torch.randn((M, K + 8), device=cuda_device, generator=gen).to(DT[dt])[:, :K]
+    w = (0.05 * torch.randn((N, K + 24), device=cuda_device, generator=gen)).to(DT[dt])[:, :K]
+    r = torch.randn((M, N + 16), device=cuda_device, generator=gen).to(DT[dt])[:, :N]
+    b = torch.randn((N,), device=cuda_device, generator=gen)
+    for epi, res in [(ops.EPI_BIAS, None), (ops.EPI_BIAS_GELU, None), (ops.EPI_BIAS_RESIDUAL, r)]:
+        y = ops.linear(x, w, b, residual=res, epilogue=epi, block_n=bn)
+        assert torch.equal(y, ops.linear(x, w, b, residual=res, epilogue=epi, block_n=-256))
+    want = x.double() @ w.double().T + b.double()
+    y = ops.linear(x, w, b, out_dtype=torch.float32, block_n=bn)
+    assert (y.double() - want).abs().max().item() < 1e-4
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
 @pytest.mark.parametrize("M,N,K,bn", [(512, 768, 768, 0), (300, 1024, 256, 192), (130, 96, 64, -64), (1000, 3072, 768, 256)])
 def test_linear_layernorm_folding(cuda_device, dt, M, N, K, bn):
     """out_stats, folded input LayerNorm and folded residual LayerNorm against the unfused oracle."""

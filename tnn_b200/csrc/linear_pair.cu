@@ -18,13 +18,13 @@ namespace lin {
 
 namespace {
 
-template <int BN, bool RES, bool FOLD>
+template <int BN, bool RES, bool FOLD, int KSUB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epi_warps<BN>(), 1)
 linear_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                    const __grid_constant__ CUtensorMap tm_y, const __grid_constant__ CUtensorMap tm_r,
                    const LinearParams p) {
     constexpr int EW = pair_epi_warps<BN>();
-    using C = PairCfg<BN, RES, FOLD, EW>;
+    using C = PairCfg<BN, RES, FOLD, EW, KSUB>;
     constexpr int STAGES = C::STAGES;
     extern __shared__ uint8_t smem_raw[];
     // Both CTAs of a pair must lay their buffers out at identical offsets: the dynamic shared-memory window starts at
@@ -75,30 +75,38 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         // into L2 (every CTA a share of the (k-block, BN/2-row) boxes), so that the first wave of tiles does not pay
         // the HBM latency on its critical path.
         const int row_boxes = (p.N + BN / 2 - 1) / (BN / 2);
-        const int boxes = p.num_k_blocks * row_boxes;
-        for (int b = blockIdx.x; b < boxes; b += gridDim.x)
-            tma_prefetch_l2_2d(&tm_w, (b % p.num_k_blocks) * BK, (b / p.num_k_blocks) * (BN / 2));
+        const int k_boxes = (p.num_k_blocks + KSUB - 1) / KSUB;
+        for (int b = blockIdx.x; b < k_boxes * row_boxes; b += gridDim.x) {
+            if (KSUB == 1) tma_prefetch_l2_2d(&tm_w, (b % k_boxes) * BK, (b / k_boxes) * (BN / 2));
+            else tma_prefetch_l2_3d(&tm_w, 0, (b / k_boxes) * (BN / 2), (b % k_boxes) * KSUB);
+        }
     }
     pdl_wait();   // x, the residual and the statistics come from earlier kernels; y may still be read by one
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer (both CTAs)
         if (elect_one()) {
-            uint32_t it = 0;
+            uint32_t st = 0, ph = 0;
             bool ok = true;
             for (int tile = pair_id; ok && tile < p.num_tiles; tile += num_pairs) {
                 const int m_blk = tile / p.num_n_tiles;
                 const int n_blk = tile % p.num_n_tiles;
-                for (int kb = 0; kb < p.num_k_blocks; ++kb, ++it) {
-                    const uint32_t s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
-                    if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag)) { ok = false; break; }
-                    uint8_t* a = smem + s * C::STAGE_BYTES;
+                const int x_row = m_blk * 256 + static_cast<int>(rank) * 128;
+                const int w_row = n_blk * BN + static_cast<int>(rank) * (BN / 2);
+                for (int kb = 0; kb < p.num_k_blocks; kb += KSUB) {
+                    if (!mbar_wait(&empty[st], ph ^ 1u, abort_flag)) { ok = false; break; }
+                    uint8_t* a = smem + st * C::STAGE_BYTES;
                     uint8_t* b = a + C::A_BYTES;
-                    if (leader) mbar_expect_tx(&full[s], 2 * C::STAGE_BYTES);
-                    const uint32_t bar = leader_addr(&full[s]);
-                    tma_load_2d_pair(a, &tm_x, bar, kb * BK, m_blk * 256 + static_cast<int>(rank) * 128);
-                    tma_load_2d_pair(b, &tm_w, bar, kb * BK, n_blk * BN + static_cast<int>(rank) * (BN / 2));
+                    if (leader) mbar_expect_tx(&full[st], 2 * C::STAGE_BYTES);
+                    const uint32_t bar = leader_addr(&full[st]);
+                    if (KSUB == 1) {
+                        tma_load_2d_pair(a, &tm_x, bar, kb * BK, x_row);
+                        tma_load_2d_pair(b, &tm_w, bar, kb * BK, w_row);
+                    } else {   // maps with K split into blocks of 64: (inside the block, row, block)
+                        tma_load_3d_pair(a, &tm_x, bar, 0, x_row, kb);
+                        tma_load_3d_pair(b, &tm_w, bar, 0, w_row, kb);
+                    }
+                    if (++st == STAGES) { st = 0; ph ^= 1u; }
                 }
             }
             if (!ok) {
@@ -109,26 +117,31 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     } else if (warp == 1) {
         // ------------------------------------------------------------ UMMA issuer (leader CTA only)
         if (leader && elect_one()) {
-            uint32_t it = 0, tcount = 0;
+            uint32_t st = 0, ph = 0, tcount = 0;
             bool ok = true;
+            const uint64_t a_desc0 = make_smem_desc_sw128(smem_u32(smem));
+            const uint64_t b_desc0 = make_smem_desc_sw128(smem_u32(smem + C::A_BYTES));
             for (int tile = pair_id; ok && tile < p.num_tiles; tile += num_pairs, ++tcount) {
                 const uint32_t buf = tcount & 1u;
                 const uint32_t aph = (tcount >> 1) & 1u;
                 if (!mbar_wait(&acc_empty[buf], aph ^ 1u, abort_flag)) { ok = false; break; }
                 tcgen05_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int kb = 0; kb < p.num_k_blocks; ++kb, ++it) {
-                    const uint32_t s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
-                    if (!mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
+                for (int kb = 0; kb < p.num_k_blocks; kb += KSUB) {
+                    if (!mbar_wait(&full[st], ph, abort_flag)) { ok = false; break; }
                     tcgen05_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + s * C::STAGE_BYTES);
-                    const uint64_t a_desc = make_smem_desc_sw128(a_addr);
-                    const uint64_t b_desc = make_smem_desc_sw128(a_addr + C::A_BYTES);
+                    const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(st * (C::STAGE_BYTES >> 4));
+                    const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(st * (C::STAGE_BYTES >> 4));
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k)
-                        umma_f16_ss_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, p.idesc, (kb | k) != 0 ? 1u : 0u);
-                    umma_commit_pair(&empty[s]);
+                    for (int sub = 0; sub < KSUB; ++sub) {
+#pragma unroll
+                        for (int k = 0; k < BK / 16; ++k)
+                            umma_f16_ss_pair(d_tmem, a_desc + static_cast<uint64_t>(sub * (C::A_BLOCK >> 4) + 2 * k),
+                                             b_desc + static_cast<uint64_t>(sub * (C::B_BLOCK >> 4) + 2 * k), p.idesc,
+                                             (kb | sub | k) != 0 ? 1u : 0u);
+                    }
+                    umma_commit_pair(&empty[st]);
+                    if (++st == STAGES) { st = 0; ph ^= 1u; }
                 }
                 if (ok) umma_commit_pair(&acc_full[buf]);
             }
@@ -193,20 +206,30 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
 
 }  // namespace
 
-template <int BN, bool RES, bool FOLD>
+template <int BN, bool RES, bool FOLD, int KSUB>
 int launch_pair(const B200LinearDesc& d, cudaStream_t stream, int sm_count) {
     constexpr int EW = pair_epi_warps<BN>();
-    using C = PairCfg<BN, RES, FOLD, EW>;
-    static_assert(C::STAGES >= 3, "pipeline too shallow");
+    using C = PairCfg<BN, RES, FOLD, EW, KSUB>;
+    static_assert(C::STAGES * KSUB >= 3 && C::STAGES >= 2, "pipeline too shallow");
     static_assert(C::COLS % 32 == 0 && EW % 4 == 0, "every epilogue warp drains whole 32-column chunks");
-    const uint64_t xd[2] = {static_cast<uint64_t>(d.K), static_cast<uint64_t>(d.M)};
-    const uint64_t xs[1] = {static_cast<uint64_t>(d.ldx) * 2};
-    const uint32_t xb[2] = {BK, 128};
-    const uint64_t wd[2] = {static_cast<uint64_t>(d.K), static_cast<uint64_t>(d.N)};
-    const uint64_t ws[1] = {static_cast<uint64_t>(d.ldw) * 2};
-    const uint32_t wb[2] = {BK, BN / 2};
     CUtensorMap tx, tw, ty, tr;
-    if (!get_tensor_map(&tx, d.x, 2, xd, xs, xb) || !get_tensor_map(&tw, d.w_nk, 2, wd, ws, wb)) return B200_ERR_DRIVER;
+    if (KSUB == 1) {
+        const uint64_t xd[2] = {static_cast<uint64_t>(d.K), static_cast<uint64_t>(d.M)};
+        const uint64_t xs[1] = {static_cast<uint64_t>(d.ldx) * 2};
+        const uint32_t xb[2] = {BK, 128};
+        const uint64_t wd[2] = {static_cast<uint64_t>(d.K), static_cast<uint64_t>(d.N)};
+        const uint64_t ws[1] = {static_cast<uint64_t>(d.ldw) * 2};
+        const uint32_t wb[2] = {BK, BN / 2};
+        if (!get_tensor_map(&tx, d.x, 2, xd, xs, xb) || !get_tensor_map(&tw, d.w_nk, 2, wd, ws, wb)) return B200_ERR_DRIVER;
+    } else {   // K as (K / 64) blocks of 64, as in linear.cu
+        const uint64_t xd[3] = {BK, static_cast<uint64_t>(d.M), static_cast<uint64_t>(d.K / BK)};
+        const uint64_t xs[2] = {static_cast<uint64_t>(d.ldx) * 2, BK * 2};
+        const uint32_t xb[3] = {BK, 128, KSUB};
+        const uint64_t wd[3] = {BK, static_cast<uint64_t>(d.N), static_cast<uint64_t>(d.K / BK)};
+        const uint64_t ws[2] = {static_cast<uint64_t>(d.ldw) * 2, BK * 2};
+        const uint32_t wb[3] = {BK, BN / 2, KSUB};
+        if (!get_tensor_map(&tx, d.x, 3, xd, xs, xb) || !get_tensor_map(&tw, d.w_nk, 3, wd, ws, wb)) return B200_ERR_DRIVER;
+    }
     ty = tx;   // placeholder when the output is fp32 (stored directly, map unused)
     if (d.out_dtype != B200_F32) {
         const uint64_t yd[2] = {static_cast<uint64_t>(d.N), static_cast<uint64_t>(d.M)};
@@ -254,14 +277,14 @@ int launch_pair(const B200LinearDesc& d, cudaStream_t stream, int sm_count) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_once.ensure(dev, []() {
-            return cudaFuncSetAttribute(linear_pair_kernel<BN, RES, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            return cudaFuncSetAttribute(linear_pair_kernel<BN, RES, FOLD, KSUB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         C::SMEM_BYTES) == cudaSuccess;
         }))
         return B200_ERR_LAUNCH;
     int pairs = max_active_pairs(BN);   // (the RES variant uses no more shared memory per CTA than its stage count allows)
     if (pairs <= 0) pairs = sm_count / 2;
     if (p.num_tiles < pairs) pairs = p.num_tiles;
-    launch_kernel(linear_pair_kernel<BN, RES, FOLD>, dim3(2 * pairs), dim3(C::THREADS), C::SMEM_BYTES, stream, tx, tw,
+    launch_kernel(linear_pair_kernel<BN, RES, FOLD, KSUB>, dim3(2 * pairs), dim3(C::THREADS), C::SMEM_BYTES, stream, tx, tw,
                   ty, tr, p);
     count_launch();
     return check_launch();
@@ -273,7 +296,7 @@ int query_pairs(int sm_count) {
     // A persistent grid must not exceed what is co-resident: a pair that cannot be placed (GPCs with an odd number
     // of free SMs) would otherwise run as a second wave after the first has finished all the work.
     using C = PairCfg<BN, false, false, pair_epi_warps<BN>()>;
-    if (cudaFuncSetAttribute(linear_pair_kernel<BN, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(linear_pair_kernel<BN, false, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              C::SMEM_BYTES) != cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -290,7 +313,7 @@ int query_pairs(int sm_count) {
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, linear_pair_kernel<BN, false, false>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, linear_pair_kernel<BN, false, false, 1>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -317,13 +340,22 @@ int max_active_pairs(int bn) {
     return cache[dev][idx] > 0 ? cache[dev][idx] : 0;
 }
 
+// k-blocks per pipeline stage for a K of whole 64-deep blocks.  A stage's hand-shake costs about as much as a 64-wide tile's
+// k-block takes, so two blocks share one there; wider tiles take longer per block, and a residual's strips leave too little
+// shared memory for double stages.  us per launch, one -> two blocks per stage: 256 x 64 tiles, 1024 rows, 3072 -> 768 with
+// residual 11.3 -> 10.2, 2048 rows, 768 -> 768 7.3 -> 6.35;  256 x 128, 2048 rows, 768 -> 2304 8.9 -> 8.4, but 3072 -> 768
+// with residual 12.7 -> 14.0;  192 and 256 wide within the noise either way.
+template <int BN, bool RES> constexpr int pair_ksub() { return BN == 64 || (BN == 128 && !RES) ? 2 : 1; }
+
 template <int BN>
 int launch_linear_pair(const B200LinearDesc& d, cudaStream_t stream, int sm_count) {
     // The TMA residual path needs 16-byte aligned residual rows (checked by the caller) and a half-precision residual.
-    const bool fold = wants_fold(d);
-    if (d.epilogue == B200_EPI_BIAS_RESIDUAL)
-        return fold ? launch_pair<BN, true, true>(d, stream, sm_count) : launch_pair<BN, true, false>(d, stream, sm_count);
-    return fold ? launch_pair<BN, false, true>(d, stream, sm_count) : launch_pair<BN, false, false>(d, stream, sm_count);
+    const bool res = d.epilogue == B200_EPI_BIAS_RESIDUAL;
+    if (wants_fold(d)) return res ? launch_pair<BN, true, true, 1>(d, stream, sm_count) : launch_pair<BN, false, true, 1>(d, stream, sm_count);
+    if (d.K % BK == 0)
+        return res ? launch_pair<BN, true, false, pair_ksub<BN, true>()>(d, stream, sm_count)
+                   : launch_pair<BN, false, false, pair_ksub<BN, false>()>(d, stream, sm_count);
+    return res ? launch_pair<BN, true, false, 1>(d, stream, sm_count) : launch_pair<BN, false, false, 1>(d, stream, sm_count);
 }
 
 template int launch_linear_pair<256>(const B200LinearDesc&, cudaStream_t, int);

@@ -11,10 +11,13 @@ namespace lin {
 // is what bounds them; more warps hide its latencies, and the register budget (128 per thread at 448 threads) holds.
 template <int BN> constexpr int pair_epi_warps() { return BN == 192 ? 12 : 8; }
 
-template <int BN, bool RES, bool FOLD, int EW = kEpiWarps>
+// KSUB = 64-deep k-blocks per pipeline stage.
+template <int BN, bool RES, bool FOLD, int EW = kEpiWarps, int KSUB = 1>
 struct PairCfg {
-    static constexpr int A_BYTES = 128 * BK * 2;          // this CTA's 128 rows of x
-    static constexpr int B_BYTES = (BN / 2) * BK * 2;     // this CTA's BN/2 rows of w
+    static constexpr int A_BLOCK = 128 * BK * 2;          // one k-block of this CTA's 128 rows of x
+    static constexpr int B_BLOCK = (BN / 2) * BK * 2;     // and of its BN/2 rows of w
+    static constexpr int A_BYTES = KSUB * A_BLOCK;
+    static constexpr int B_BYTES = KSUB * B_BLOCK;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     // output staging strips (TMA store); with RES two per warp, which also receive the residual tile (TMA load)
     static constexpr int EPI_WARPS = EW;
@@ -49,6 +52,13 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(leader_bar), "r"(c0), "r"(c1)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, uint32_t leader_bar, int32_t c0,
+                                                 int32_t c1, int32_t c2) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(leader_bar), "r"(c0), "r"(c1), "r"(c2)
         : "memory");
 }
 __device__ __forceinline__ void umma_f16_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
