@@ -300,13 +300,14 @@ int launch_linear(const B200LinearDesc& d, cudaStream_t stream, int sm_count) {
     return launch_linear_t<128, BN, 1, STAGES, false>(d, stream, sm_count);
 }
 
-// Tile choice.  Estimated time ~ waves * (columns per tile * cost per column + fixed per-tile cost), in units of
-// "accumulator columns per SM".  What bounds a k-block is the slower of the tensor pipe (2 clocks per accumulator
-// column for a 256-row pair tile) and the SM's read port from L2 (64 bytes per clock: every SM of a pair fetches 128
-// rows of x and BN/2 rows of w per k-block, (128 + BN/2) * 128 bytes): 512 | 512 clocks for BN = 256, 384 | 448 for 192,
-// 256 | 384 for 128, 128 | 320 for 64 — the profile of the 256-wide tile shows 11.3 TB/s from L2 to the SMs, 80 % of
-// 148 ports, at 89 % tensor-pipe activity.  Hence the cost per column rises as tiles narrow.  Single-CTA tiles
-// (128 x BN) fetch BN rows of w per SM and k-block.
+// Tile choice.  Estimated time ~ waves * (columns per tile * cost per column + fixed per-tile cost) + tail, in units of
+// "accumulator columns per SM": a k-block of a 256-wide pair tile, 512 clocks of the tensor pipe and of the SM's read port from
+// L2 alike, is 256 of them.  The costs per column are fitted to measured times per k-block (540, 448, 327 and 267 clocks
+// for pair tiles 256, 192, 128 and 64 wide) and per wave at K = 768 (256 wide 4.4-5.0 us, 192 wide 3.5-4.1); narrower tiles fetch
+// more rows of x per flop.  The tail is the last tile's epilogue, which nothing hides: 128 columns per warp on 256-wide tiles,
+// 64 on 192- and 128-wide ones; it weighs less the longer the mainloop.  Against costs without a tail that had 256-wide tiles
+// up to 3 % too cheap: 768 -> 3072 + GELU at 8192 rows 33.9 -> 31.6 us (192 wide), at 4096 rows 18.5 -> 17.5, 768 -> 2304 at
+// 2048 rows 8.9 -> 8.4 (128 wide).  With many waves the choice is as before.
 struct TileChoice {
     bool pair;
     int bn;
@@ -332,15 +333,17 @@ TileChoice choose_tile(const B200LinearDesc& d, int sm_count) {
     }
     TileChoice best = {false, 128};
     double best_t = 1e300;
+    const double k_blocks = static_cast<double>((d.K + BK - 1) / BK);
+    auto tail = [&](int bn) { return (bn == 256 ? 200.0 : (bn == 64 ? 50.0 : 100.0)) * 12.0 / k_blocks; };
     if (M > 128) {
         const int bns[4] = {256, 192, 128, 64};
-        const double cost[4] = {1.0, 1.17, 1.50, 2.50};
+        const double cost[4] = {1.0, 1.05, 1.28, 2.10};
         for (int i = 0; i < 4; ++i) {
             int pairs = max_active_pairs(bns[i]);
             if (pairs <= 0) continue;
             const int64_t tiles = ((M + 255) / 256) * ((N + bns[i] - 1) / bns[i]);
             const int64_t waves = (tiles + pairs - 1) / pairs;
-            const double t = static_cast<double>(waves) * (bns[i] * cost[i] + 16.0);
+            const double t = static_cast<double>(waves) * (bns[i] * cost[i] + 16.0) + tail(bns[i]);
             if (t < best_t) {
                 best_t = t;
                 best = {true, bns[i], 128};
@@ -352,7 +355,7 @@ TileChoice choose_tile(const B200LinearDesc& d, int sm_count) {
     for (int i = 0; i < 3; ++i) {
         const int64_t tiles = ((M + BM - 1) / BM) * ((N + bns1[i] - 1) / bns1[i]);
         const int64_t waves = (tiles + sm_count - 1) / sm_count;
-        const double t = static_cast<double>(waves) * (bns1[i] * cost1[i] + 16.0);
+        const double t = static_cast<double>(waves) * (bns1[i] * cost1[i] + 16.0) + tail(bns1[i]);
         if (t < best_t) {
             best_t = t;
             best = {false, bns1[i], 128};
