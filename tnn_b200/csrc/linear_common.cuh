@@ -10,7 +10,6 @@ namespace lin {
 constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int kEpiWarps = 8;
-constexpr int kThreads = 64 + kEpiWarps * 32;
 
 struct LinearParams {
     const float* bias;
