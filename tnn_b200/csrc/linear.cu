@@ -42,7 +42,8 @@ struct Cfg {
     static_assert((2 * STAGES + 4) * 8 + 8 <= 512, "barriers");
 };
 
-template <int TM, int BN, int KSUB, int STAGES, bool FOLD>
+// FEW: the whole launch has fewer rows than TM (p.x_rows of them in a load box).
+template <int TM, int BN, int KSUB, int STAGES, bool FOLD, bool FEW>
 __global__ void __launch_bounds__(Cfg<TM, BN, KSUB, STAGES, FOLD>::THREADS, 1)
 linear_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
               const __grid_constant__ CUtensorMap tm_y, const LinearParams p) {
@@ -98,6 +99,7 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
         if (elect_one()) {
             uint32_t st = 0, ph = 0;
             bool ok = true;
+            const uint32_t stage_tx = FEW ? static_cast<uint32_t>(KSUB * p.x_rows * BK * 2 + C::B_BYTES) : C::STAGE_BYTES;
             for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x) {
                 const int m_blk = tile / p.num_n_tiles;
                 const int n_blk = tile % p.num_n_tiles;
@@ -105,7 +107,7 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
                     if (!mbar_wait(&empty[st], ph ^ 1u, abort_flag)) { ok = false; break; }
                     uint8_t* a = smem + st * C::STAGE_BYTES;
                     uint8_t* b = a + C::A_BYTES;
-                    mbar_expect_tx(&full[st], C::STAGE_BYTES);
+                    mbar_expect_tx(&full[st], stage_tx);
                     if (KSUB == 1) {
                         tma_load_2d(a, &tm_x, &full[st], kb * BK, m_blk * TM);
                         tma_load_2d(b, &tm_w, &full[st], kb * BK, n_blk * BN);
@@ -127,6 +129,8 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
         if (elect_one()) {
             uint32_t st = 0, ph = 0, tcount = 0;
             bool ok = true;
+            // (with fewer rows than TM the UMMA reads on into whatever follows a k-block in the stage: rows that are not stored)
+            const uint64_t a_step = static_cast<uint64_t>(FEW ? p.x_rows * BK * 2 : C::A_BLOCK) >> 4;
             const uint64_t a_desc0 = make_smem_desc_sw128(smem_u32(smem));
             const uint64_t b_desc0 = make_smem_desc_sw128(smem_u32(smem + C::A_BYTES));
             for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x, ++tcount) {
@@ -145,7 +149,7 @@ linear_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
 #pragma unroll
                         for (int k = 0; k < BK / 16; ++k) {
                             // 16 elements along K = 32 bytes inside the 128-byte swizzled row: +2 in (address >> 4) units
-                            umma_f16_ss(d_tmem, a_desc + static_cast<uint64_t>(sub * (C::A_BLOCK >> 4) + 2 * k),
+                            umma_f16_ss(d_tmem, a_desc + static_cast<uint64_t>(sub) * a_step + static_cast<uint64_t>(2 * k),
                                         b_desc + static_cast<uint64_t>(sub * (C::B_BLOCK >> 4) + 2 * k), p.idesc,
                                         (kb | sub | k) != 0 ? 1u : 0u);
                         }
@@ -219,9 +223,11 @@ int device_sm_count() {
     return v;
 }
 
-template <int TM, int BN, int KSUB, int STAGES, bool FOLD>
+template <int TM, int BN, int KSUB, int STAGES, bool FOLD, bool FEW = false>
 int launch_linear_t(const B200LinearDesc& d, cudaStream_t stream, int sm_count) {
     using C = Cfg<TM, BN, KSUB, STAGES, FOLD>;
+    const int x_rows = FEW ? static_cast<int>((d.M + 7) / 8 * 8) : TM;
+    if (x_rows > TM || (FEW && KSUB == 1)) return B200_ERR_PARAM;
     CUtensorMap tx, tw, ty;
     if (KSUB == 1) {
         const uint64_t xd[2] = {static_cast<uint64_t>(d.K), static_cast<uint64_t>(d.M)};
@@ -236,7 +242,7 @@ int launch_linear_t(const B200LinearDesc& d, cudaStream_t stream, int sm_count) 
         // land one behind the other, each in the layout the UMMA descriptors expect.  Blocks beyond K read as zeros.
         const uint64_t xd[3] = {BK, static_cast<uint64_t>(d.M), static_cast<uint64_t>(d.K / BK)};
         const uint64_t xs[2] = {static_cast<uint64_t>(d.ldx) * 2, BK * 2};
-        const uint32_t xb[3] = {BK, TM, KSUB};
+        const uint32_t xb[3] = {BK, static_cast<uint32_t>(x_rows), KSUB};
         const uint64_t wd[3] = {BK, static_cast<uint64_t>(d.N), static_cast<uint64_t>(d.K / BK)};
         const uint64_t ws[2] = {static_cast<uint64_t>(d.ldw) * 2, BK * 2};
         const uint32_t wb[3] = {BK, BN, KSUB};
@@ -277,17 +283,18 @@ int launch_linear_t(const B200LinearDesc& d, cudaStream_t stream, int sm_count) 
     p.ln_eps = d.ln_eps;
     p.k_slots = (p.K + 31) / 32;
     p.n_slots = (p.N + 31) / 32;
+    p.x_rows = x_rows;
 
     static PerDeviceOnce attr_once;
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_once.ensure(dev, []() {
-            return cudaFuncSetAttribute(linear_kernel<TM, BN, KSUB, STAGES, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            return cudaFuncSetAttribute(linear_kernel<TM, BN, KSUB, STAGES, FOLD, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         C::SMEM_BYTES) == cudaSuccess;
         }))
         return B200_ERR_LAUNCH;
     const int grid = p.num_tiles < sm_count ? p.num_tiles : sm_count;
-    launch_kernel(linear_kernel<TM, BN, KSUB, STAGES, FOLD>, dim3(grid), dim3(C::THREADS), C::SMEM_BYTES, stream, tx, tw, ty, p);
+    launch_kernel(linear_kernel<TM, BN, KSUB, STAGES, FOLD, FEW>, dim3(grid), dim3(C::THREADS), C::SMEM_BYTES, stream, tx, tw, ty, p);
     count_launch();
     return check_launch();
 }
@@ -413,8 +420,12 @@ extern "C" int b200_linear_fwd(const B200LinearDesc* d, b200_stream_t stream_) {
         }
     }
     if (tc.tm == 64) {
-        return tc.bn == 32 ? launch_linear_t<64, 32, 4, 4, false>(*d, stream, sms)
-                           : launch_linear_t<64, 64, 4, 3, false>(*d, stream, sms);
+        if (tc.bn == 64) return launch_linear_t<64, 64, 4, 3, false>(*d, stream, sms);
+        // Up to 48 rows fetch only the rows that exist, rounded up to the swizzle's eight: rows beyond M cross the SM's read
+        // port from L2 as zeros.  us per launch at 16 rows: 768 -> 2304 3.8 -> 3.2, 768 -> 3072 4.6 -> 3.5; at 41 rows 768 -> 3072
+        // 3.95 -> 3.75; at 56 rows and more there is nothing left to gain.
+        return d->M <= 48 ? launch_linear_t<64, 32, 4, 4, false, true>(*d, stream, sms)
+                          : launch_linear_t<64, 32, 4, 4, false>(*d, stream, sms);
     }
     switch (tc.bn) {
         case 256: return launch_linear<256, 4, 1, 4>(*d, stream, sms);

@@ -31,6 +31,7 @@ struct LinearParams {
     const float* res_ln_beta;
     float ln_eps;
     int k_slots, n_slots;   // ceil(K/32), ceil(N/32)
+    int x_rows;             // single-CTA tiles: rows of x in a load box (the tile's, or fewer if there are no more)
 };
 
 
