@@ -18,14 +18,18 @@ def _require_cuda(*ts):
             raise ValueError("tnn_b200 operators take CUDA tensors only (there is no CPU path)")
 
 
-def _rows(t, width):
+def _rows(t, width, at_least=0):
     """`t` as rows of `width` elements: (tensor that holds them, number of rows, row stride).  A contiguous tensor, the
-    usual one, needs no view of its own: making views costs more than filling a descriptor."""
-    if t.is_contiguous():
-        return t, t.numel() // width, width
-    t2 = t.reshape(-1, width)
-    assert t2.stride(1) == 1
-    return t2, t2.shape[0], t2.stride(0)
+    usual one, needs no view of its own: making views costs more than filling a descriptor.  What does not divide into
+    such rows is refused by `reshape`; so are fewer than `at_least` rows, which a kernel would reach beyond."""
+    if t.is_contiguous() and width and t.numel() % width == 0:
+        rows, ld = t.numel() // width, width
+    else:
+        t = t.reshape(-1, width)
+        assert t.stride(1) == 1
+        rows, ld = t.shape[0], t.stride(0)
+    assert rows >= at_least, "fewer rows than the input has"
+    return t, rows, ld
 
 
 def pack_weight(w_kn, dtype=torch.float16, out=None):
@@ -84,12 +88,12 @@ def _linear_desc(x, w_nk, bias, residual, epilogue, out_dtype, out, block_n, out
     x2, M, ldx = _rows(x, K)
     if out is None:
         out = torch.empty(x.shape[:-1] + (N,), dtype=out_dtype or x.dtype, device=x.device)
-    y2, _, ldy = _rows(out, N)
+    y2, _, ldy = _rows(out, N, M)
     d = capi.LinearDesc(x2.data_ptr(), w_nk.data_ptr(), capi.ptr(bias), None, y2.data_ptr(), M, N, K, ldx,
                         w_nk.stride(0), 0, ldy, capi.dtype_code(x.dtype), capi.dtype_code(out.dtype), epilogue, block_n)
     if residual is not None:
         assert residual.dtype == x.dtype
-        r2, _, d.ldr = _rows(residual, N)
+        r2, _, d.ldr = _rows(residual, N, M)
         d.residual = r2.data_ptr()
     # LayerNorm folding: ln_in = (stats of x, c1, c2); res_ln = (stats of residual, gamma, beta)
     d.ln_eps = float(ln_eps)
@@ -157,12 +161,12 @@ def _layernorm_desc(x, gamma, beta, eps, residual, out_dtype, out):
     x2, rows, ldx = _rows(x, H)
     if out is None:
         out = torch.empty(x.shape, dtype=out_dtype or x.dtype, device=x.device)
-    y2, _, ldy = _rows(out, H)
+    y2, _, ldy = _rows(out, H, rows)
     d = capi.LayerNormDesc(x2.data_ptr(), None, gamma.data_ptr(), beta.data_ptr(), y2.data_ptr(), rows, H, ldx, 0, ldy,
                            capi.dtype_code(x.dtype), capi.dtype_code(out.dtype), float(eps))
     if residual is not None:
         assert residual.dtype == x.dtype
-        r2, _, d.ldr = _rows(residual, H)
+        r2, _, d.ldr = _rows(residual, H, rows)
         d.residual = r2.data_ptr()
     return d, out
 
