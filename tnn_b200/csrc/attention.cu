@@ -265,13 +265,13 @@ attention_pingpong_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                     for (int k = 0; k < HD / 16; ++k)
                         umma_f16_ss(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc_qk, k != 0 ? 1u : 0u);
                     umma_commit(&s_full[wg]);
+                    umma_commit(&k_empty[st]);   // by the lane that issued the UMMAs: a commit covers its own thread's only
                 }
                 __syncwarp();
             };
             // Per key tile j and warpgroup w: as soon as the warpgroup holds S_w(j) in registers, S_w(j+1) is issued;
-            // when it has written P_w(j), P_w V(j) follows.  `last` = this is the CTA's last warpgroup: its commits
-            // release the K / V stages.
-            auto step_s = [&](auto wg_c, const int j, const bool last) -> bool {
+            // when it has written P_w(j), P_w V(j) follows.  The commits of both warps release the K / V stages.
+            auto step_s = [&](auto wg_c, const int j) -> bool {
                 constexpr int wg = decltype(wg_c)::value;
                 if (j + 1 >= n_tiles) return true;
                 const int st_next = (j + 1) % PP_NST;
@@ -279,10 +279,9 @@ attention_pingpong_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 if (!mbar_wait(&k_full[st_next], (static_cast<uint32_t>(j + 1) / PP_NST) & 1u, abort_flag)) return false;
                 tcgen05_fence_after();
                 issue_s(wg_c, st_next);
-                if (last && lane == 0) umma_commit(&k_empty[st_next]);
                 return true;
             };
-            auto step_pv = [&](auto wg_c, const int j, const bool last) -> bool {
+            auto step_pv = [&](auto wg_c, const int j) -> bool {
                 constexpr int wg = decltype(wg_c)::value;
                 const int st = j % PP_NST;
                 if (!mbar_wait(&p_full[wg], static_cast<uint32_t>(j) & 1u, abort_flag)) return false;
@@ -300,7 +299,7 @@ attention_pingpong_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                         umma_f16_ts(d_tmem, a_tmem + k * 8, b_desc + static_cast<uint64_t>(k * (2048 >> 4)), idesc_pv,
                                     k != 0 ? 1u : acc0);
                     umma_commit(&o_full[wg]);
-                    if (last) umma_commit(&v_empty[st]);
+                    umma_commit(&v_empty[st]);
                 }
                 __syncwarp();
                 return true;
@@ -311,11 +310,10 @@ attention_pingpong_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                 if (ok) {
                     tcgen05_fence_after();
                     issue_s(wg_c, 0);
-                    if (lane == 0) umma_commit(&k_empty[0]);
                 }
                 for (int j = 0; ok && j < n_tiles; ++j) {
-                    ok = step_s(wg_c, j, true);
-                    if (ok) ok = step_pv(wg_c, j, true);
+                    ok = step_s(wg_c, j);
+                    if (ok) ok = step_pv(wg_c, j);
                     ok = __all_sync(0xffffffffu, ok);
                 }
             };
