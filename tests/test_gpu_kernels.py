@@ -304,6 +304,29 @@ def test_attention_of_a_batch_equals_its_sequences_alone(cuda_device, S):
         assert torch.equal(ops.attention(qkv, heads, mask, kv), alone)
 
 
+@pytest.mark.parametrize("S,dt", [(896, "f16"), (896, "bf16"), (1000, "f16"), (1024, "f16"), (1152, "f16"), (2048, "bf16")])
+def test_attention_beyond_768_tokens(cuda_device, S, dt):
+    """769 .. 1024 tokens: the persistent kernel whose issuing warps run as whole warps, three and more items per CTA; at
+    896 the last query block has one tile, at 1000 its second one is partly empty.  Beyond: one item per CTA, the K/V ring
+    goes round two to four times.  Ragged lengths; every sequence against 64-bit softmax, and bit for bit what it gives alone."""
+    B, heads = 28, 4
+    gen = torch.Generator(device=cuda_device).manual_seed(S)
+    qkv = torch.randn((B, S, 3 * heads * 64), device=cuda_device, generator=gen).to(DT[dt])
+    lens = torch.randint(1, S + 1, (B,), device=cuda_device, generator=gen)
+    lens[0], lens[1] = S, 1
+    mask = torch.where(torch.arange(S, device=cuda_device)[None] < lens[:, None], 0.0, -10000.0).contiguous()
+    kv = ops.mask_to_kv_len(mask)
+    got = ops.attention(qkv, heads, mask, kv)
+    for b in range(B):
+        q, k, v = (qkv[b, :, i * heads * 64:(i + 1) * heads * 64].double().reshape(S, heads, 64).transpose(0, 1) for i in range(3))
+        n = int(lens[b])
+        want = (torch.softmax(q @ k[:, :n].transpose(1, 2) * 0.125, -1) @ v[:, :n]).transpose(0, 1).reshape(S, heads * 64)
+        assert (got[b].double() - want).abs().max().item() < (6e-3 if dt == "f16" else 3e-2), (b, n)
+    alone = torch.cat([ops.attention(qkv[b:b + 1], heads, mask[b:b + 1], kv[b:b + 1]) for b in range(B)])
+    for _ in range(5):
+        assert torch.equal(ops.attention(qkv, heads, mask, kv), alone)
+
+
 @pytest.mark.parametrize("S,lengths", [(256, [77, 200]), (128, [5, 100]), (96, [33, 96])])
 def test_attention_padded_keys_have_exactly_zero_weight(cuda_device, S, lengths):
     """Perturbing K/V rows of padded keys must leave every output bit-identical."""
