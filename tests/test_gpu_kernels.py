@@ -110,6 +110,29 @@ def test_linear_one_wave_tiles(cuda_device, dt, M, N, K):
 
 
 @pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("M,N,K,bn", [
+    (2500, 3080, 320, -128), (2500, 3080, 320, -64),   # stages of two k-blocks, an odd number of them, three and more tiles per CTA
+    (2500, 3080, 576, -64), (41, 30520, 576, -128),
+    (200, 2312, 576, 0), (300, 3080, 576, 0), (520, 3000, 832, 0),      # chosen: 64 x 64, 128 x 64, 128 x 128 in one wave
+    (300, 3080, 448, 0), (520, 3000, 448, 0), (2100, 3080, 448, 0),     # seven k-blocks: one per stage, one and several waves
+    (41, 30520, 576, 0), (384, 776, 64, 0), (41, 768, 128, 0),
+])
+def test_linear_rings_carried_from_tile_to_tile(cuda_device, dt, M, N, K, bn):
+    """Single-CTA tiles whose ring goes on from a half-filled last stage into the next tile, and both sides of the chooser's
+    lines (k-blocks, waves), bit for bit as 128 x 256 tiles with one k-block per stage give it and against 64 bits."""
+    gen = torch.Generator(device=cuda_device).manual_seed(M + N + K)
+    x = torch.randn((M, K), device=cuda_device, generator=gen).to(DT[dt])
+    w = (0.05 * torch.randn((N, K), device=cuda_device, generator=gen)).to(DT[dt])
+    r = torch.randn((M, N), device=cuda_device, generator=gen).to(DT[dt])
+    b = torch.randn((N,), device=cuda_device, generator=gen)
+    for epi, res in [(ops.EPI_BIAS, None), (ops.EPI_BIAS_GELU, None), (ops.EPI_BIAS_RESIDUAL, r)]:
+        y = ops.linear(x, w, b, residual=res, epilogue=epi, block_n=bn)
+        assert torch.equal(y, ops.linear(x, w, b, residual=res, epilogue=epi, block_n=-256))
+    y = ops.linear(x, w, b, out_dtype=torch.float32, block_n=bn)
+    assert (y.double() - (x.double() @ w.double().T + b.double())).abs().max().item() < 1e-4   # fp32 sums, as above
+
+
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
 @pytest.mark.parametrize("bn", [64, 128])
 @pytest.mark.parametrize("M,N,K", [(129, 72, 64), (300, 200, 320), (257, 776, 1088), (2500, 776, 192), (300, 200, 328)])
 def test_linear_pair_tiles_with_two_k_blocks_per_stage(cuda_device, dt, bn, M, N, K):

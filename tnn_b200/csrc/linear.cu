@@ -301,73 +301,80 @@ int launch_linear_t(const B200LinearDesc& d, cudaStream_t stream, int sm_count) 
 
 // KSUB / KSTAGES: the multi-block pipeline, for a K of whole 64-deep blocks (its maps split K into such blocks).
 template <int BN, int STAGES, int KSUB, int KSTAGES>
-int launch_linear(const B200LinearDesc& d, cudaStream_t stream, int sm_count) {
+int launch_linear(const B200LinearDesc& d, cudaStream_t stream, int sm_count, bool multi_block) {
     if (wants_fold(d)) return launch_linear_t<128, BN, 1, STAGES - 1, true>(d, stream, sm_count);
-    if (KSUB > 1 && d.K % BK == 0) return launch_linear_t<128, BN, KSUB, KSTAGES, false>(d, stream, sm_count);
+    if (KSUB > 1 && multi_block) return launch_linear_t<128, BN, KSUB, KSTAGES, false>(d, stream, sm_count);
     return launch_linear_t<128, BN, 1, STAGES, false>(d, stream, sm_count);
 }
 
-// Tile choice.  Estimated time ~ waves * (columns per tile * cost per column + fixed per-tile cost) + tail, in units of
-// "accumulator columns per SM": a k-block of a 256-wide pair tile, 512 clocks of the tensor pipe and of the SM's read port from
-// L2 alike, is 256 of them.  The costs per column are fitted to measured times per k-block (540, 448, 327 and 267 clocks
-// for pair tiles 256, 192, 128 and 64 wide) and per wave at K = 768 (256 wide 4.4-5.0 us, 192 wide 3.5-4.1); narrower tiles fetch
-// more rows of x per flop.  The tail is the last tile's epilogue, which nothing hides: 128 columns per warp on 256-wide tiles,
-// 64 on 192- and 128-wide ones; it weighs less the longer the mainloop.  Against costs without a tail that had 256-wide tiles
-// up to 3 % too cheap: 768 -> 3072 + GELU at 8192 rows 33.9 -> 31.6 us (192 wide), at 4096 rows 18.5 -> 17.5, 768 -> 2304 at
-// 2048 rows 8.9 -> 8.4 (128 wide).  With many waves the choice is as before.
+// Tile choice.  With few tiles a launch is one tile's serial chain (one-wave rules below); beyond, estimated time ~ waves *
+// (columns per tile * cost per column + fixed per-tile cost) + tail, in units of accumulator columns per SM.
 struct TileChoice {
     bool pair;
     int bn;
-    int tm = 128;   // rows of a single-CTA tile
+    int tm = 128;               // rows of a single-CTA tile
+    bool multi_block = false;   // several k-blocks per pipeline stage where the tile has such a form (K of whole blocks)
 };
 TileChoice choose_tile(const B200LinearDesc& d, int sm_count) {
     const int64_t M = d.M, N = d.N;
+    const int64_t k_blocks = (d.K + BK - 1) / BK;
+    const bool whole = !wants_fold(d) && d.K % BK == 0;
+    // Stages of several k-blocks pay from about eight blocks on (us per launch at 512, 320, 128 deep, one block -> several:
+    // 128 x 64 tiles, 768 columns + residual, 512 rows 4.43 -> 4.32 at 512, 3.38 -> 3.41 at 128; 2304 columns, 256 rows 3.63 ->
+    // 3.66 at 320; 128 x 128, 2304 columns, 1024 rows 4.22 -> 4.57 at 320): a shorter chain is over before the ring is full.
+    const bool deep = whole && k_blocks >= 8;
+    auto tiles = [&](int64_t tm, int64_t tn) { return ((M + tm - 1) / tm) * ((N + tn - 1) / tn); };
     // Few rows: a launch is bound by its latencies (hand-over, first loads, the serial chain of k-blocks of one tile, drain),
     // so the smallest tile that still fits one wave is the fastest: the more SMs fetch operands at once, the shorter each
-    // one's chain.  12 launches in turn on weights of their own, us per launch, before (128 x 64 tiles, one k-block per
-    // stage) -> on the tile below:  M = 41: 768 -> 768 4.8 -> 3.5, 768 -> 2304 4.6 -> 3.4, 768 -> 3072 4.9 -> 4.0,
-    // 3072 -> 768 11.1 -> 6.3;  M = 256: 5.1 -> 3.7, 4.9 -> 4.2, 5.4 -> 5.1, 11.7 -> 6.8;  M = 1024: 768 -> 768 5.4 -> 5.1,
-    // 3072 -> 768 12.7 -> 10.7 (128 x 64).  One tile more than SMs and the next wider one is ahead: 768 -> 3072 at 128 rows
+    // one's chain.  12 launches in turn on weights of their own, us per launch, 128 x 64 tiles with one k-block per
+    // stage -> the tile below:  M = 41: 768 -> 768 5.4 -> 3.5, 768 -> 2304 4.7 -> 3.4, 768 -> 3072 5.1 -> 3.8,
+    // 3072 -> 768 13.3 -> 7.7;  M = 256: 5.9 -> 3.7, 5.0 -> 4.2, 5.5 -> 5.1, 12.5 -> 7.1;  M = 1024: 768 -> 768 5.9 -> 5.1,
+    // 3072 -> 768 13.1 -> 10.7 (128 x 64).  One tile more than SMs and the next wider one is ahead: 768 -> 3072 at 128 rows
     // 4.9 on 192 tiles of 64 x 32, 4.5 on 96 of 64 x 64.  All tiles add a row's products up in the same order, so the choice
     // changes no bit of the result.
-    if (!wants_fold(d) && d.K % BK == 0) {
-        const struct { int tm, bn; } small[3] = {{64, 32}, {64, 64}, {128, 64}};
-        for (const auto& t : small)
-            if (((M + t.tm - 1) / t.tm) * ((N + t.bn - 1) / t.bn) <= sm_count) return {false, t.bn, t.tm};
-        // 128 x 128 drains two chunks per warp, and a residual of the second is not fetched ahead: 768 -> 2304 at 1024 rows
-        // 5.9 against 6.4 us on pair tiles, 768 -> 768 with a residual at 2048 rows 8.1 against 6.7.
-        if (d.epilogue != B200_EPI_BIAS_RESIDUAL && ((M + 127) / 128) * ((N + 127) / 128) <= sm_count) return {false, 128};
-    }
-    TileChoice best = {false, 128};
+    if (whole && k_blocks >= 2 && tiles(64, 32) <= sm_count) return {false, 32, 64};   // (64 deep: 2.6 us on 128 x 64, 3.2 on these)
+    if (deep && tiles(64, 64) <= sm_count) return {false, 64, 64};
+    if (whole && tiles(128, 64) <= sm_count) return {false, 64, 128, deep};
+    // 128 x 128 drains two chunks per warp, and a residual of the second is not fetched ahead: 768 -> 2304 at 1024 rows
+    // 5.8 against 6.5 us on pair tiles, 768 -> 768 with a residual at 2048 rows 7.8 against 6.7.  A k-block takes it longer
+    // than a pair tile: 1024 deep still ahead (768 rows, 3072 columns: 6.7 against 7.2), 3072 deep behind (6144 rows, 256
+    // columns: 13.5 against 12.8).
+    if (whole && k_blocks <= 16 && d.epilogue != B200_EPI_BIAS_RESIDUAL && tiles(128, 128) <= sm_count)
+        return {false, 128, 128, deep};
+
+    // More than one wave.  Costs per column relative to 256-wide pair tiles, for pair tiles 256, 192, 128, 64 and single-CTA
+    // tiles 256, 128, 64 wide; the narrower ones fetch more rows of x per flop and hand more stages over.  For a deep K they
+    // are fitted to the measured choice between tiles at 129 .. 65536 rows, 768- and 1024-wide models; GELU hides better
+    // behind 192-wide tiles' twelve epilogue warps.  The tail is the last tile's epilogue, which nothing hides: 128 columns per
+    // warp on 256-wide tiles, 64 on 192- and 128-wide ones; it weighs less the longer the mainloop.  us per launch, 256 wide ->
+    // chosen: 768 -> 3072 + GELU at 4096 rows 18.6 -> 17.7, 5120 23.6 -> 20.9, 8192 32.9 -> 30.5, 16384 63.4 -> 61.4;  768 -> 2304
+    // at 2048 rows 8.9 -> 8.5 (128 wide);  768 -> 768 + residual at 16384 rows 21.4 -> 19.4, 32768 39.9 -> 38.5;  1024 -> 3072 at
+    // 5120 rows 25.7 -> 24.3.  Where the 256-wide tile stays ahead, 192 wide: 1024 -> 3072 at 16384 rows 74.7 | 76.5, at 10240
+    // 46.5 | 48.0;  768 -> 768 + residual at 65536 rows 75.6 | 76.4.
+    // Otherwise (a short K, a K that is not in whole blocks, LayerNorm folding: one k-block per stage) narrow tiles cost more and
+    // a tail says nothing: 776 -> 3072 + GELU at 4096 rows 24.2 us on 256-, 25.7 on 192-wide tiles, 776 -> 768 + residual
+    // at 5120 rows 13.2 | 14.8 on 128-wide ones.
+    const double pair_cost[2][4] = {{1.0, 1.17, 1.50, 2.50}, {1.0, d.epilogue == B200_EPI_BIAS_GELU ? 1.05 : 1.10, 1.28, 2.10}};
+    const double single_cost[3] = {1.35, 1.50, 1.90};
+    auto tail = [&](int bn) {
+        if (!deep || M <= 128) return 0.0;   // (up to 128 rows only single-CTA tiles compete, and the weights' bytes decide)
+        return (bn == 256 ? 200.0 : (bn == 64 ? 50.0 : 100.0)) * 12.0 / static_cast<double>(k_blocks);
+    };
+    TileChoice best = {false, 128, 128, deep};
     double best_t = 1e300;
-    const double k_blocks = static_cast<double>((d.K + BK - 1) / BK);
-    auto tail = [&](int bn) { return (bn == 256 ? 200.0 : (bn == 64 ? 50.0 : 100.0)) * 12.0 / k_blocks; };
-    if (M > 128) {
-        const int bns[4] = {256, 192, 128, 64};
-        const double cost[4] = {1.0, 1.05, 1.28, 2.10};
-        for (int i = 0; i < 4; ++i) {
-            int pairs = max_active_pairs(bns[i]);
-            if (pairs <= 0) continue;
-            const int64_t tiles = ((M + 255) / 256) * ((N + bns[i] - 1) / bns[i]);
-            const int64_t waves = (tiles + pairs - 1) / pairs;
-            const double t = static_cast<double>(waves) * (bns[i] * cost[i] + 16.0) + tail(bns[i]);
-            if (t < best_t) {
-                best_t = t;
-                best = {true, bns[i], 128};
-            }
-        }
-    }
-    const int bns1[3] = {256, 128, 64};
-    const double cost1[3] = {1.35, 1.50, 1.90};
-    for (int i = 0; i < 3; ++i) {
-        const int64_t tiles = ((M + BM - 1) / BM) * ((N + bns1[i] - 1) / bns1[i]);
-        const int64_t waves = (tiles + sm_count - 1) / sm_count;
-        const double t = static_cast<double>(waves) * (bns1[i] * cost1[i] + 16.0) + tail(bns1[i]);
+    auto consider = [&](bool pair, int bn, int64_t n_tiles, int64_t slots, double cost) {
+        const double t = static_cast<double>((n_tiles + slots - 1) / slots) * (bn * cost + 16.0) + tail(bn);
         if (t < best_t) {
             best_t = t;
-            best = {false, bns1[i], 128};
+            best = {pair, bn, 128, deep};
         }
+    };
+    const int pair_bn[4] = {256, 192, 128, 64}, single_bn[3] = {256, 128, 64};
+    for (int i = 0; i < 4 && M > 128; ++i) {
+        const int pairs = max_active_pairs(pair_bn[i]);
+        if (pairs > 0) consider(true, pair_bn[i], tiles(256, pair_bn[i]), pairs, pair_cost[deep ? 1 : 0][i]);
     }
+    for (int i = 0; i < 3; ++i) consider(false, single_bn[i], tiles(128, single_bn[i]), sm_count, single_cost[i]);
     return best;
 }
 
@@ -402,20 +409,21 @@ extern "C" int b200_linear_fwd(const B200LinearDesc* d, b200_stream_t stream_) {
     const int sms = device_sm_count();
     if (sms <= 0) return B200_ERR_NOT_SM100;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    const bool whole = d->K % BK == 0;
     TileChoice tc;
     if (d->block_n == 0) {
         tc = choose_tile(*d, sms);
     } else if (d->block_n > 0) {
-        tc = {d->M > 128, d->block_n, 128};
+        tc = {d->M > 128, d->block_n, 128, whole};
     } else {
-        tc = {false, -d->block_n, 128};
+        tc = {false, -d->block_n, 128, whole};
     }
     if (tc.pair) {
         switch (tc.bn) {
-            case 256: return launch_linear_pair<256>(*d, stream, sms);
-            case 192: return launch_linear_pair<192>(*d, stream, sms);
-            case 128: return launch_linear_pair<128>(*d, stream, sms);
-            case 64: return launch_linear_pair<64>(*d, stream, sms);
+            case 256: return launch_linear_pair<256>(*d, stream, sms, tc.multi_block);
+            case 192: return launch_linear_pair<192>(*d, stream, sms, tc.multi_block);
+            case 128: return launch_linear_pair<128>(*d, stream, sms, tc.multi_block);
+            case 64: return launch_linear_pair<64>(*d, stream, sms, tc.multi_block);
             default: return B200_ERR_PARAM;
         }
     }
@@ -428,9 +436,9 @@ extern "C" int b200_linear_fwd(const B200LinearDesc* d, b200_stream_t stream_) {
                           : launch_linear_t<64, 32, 4, 4, false>(*d, stream, sms);
     }
     switch (tc.bn) {
-        case 256: return launch_linear<256, 4, 1, 4>(*d, stream, sms);
-        case 128: return launch_linear<128, 6, 2, 3>(*d, stream, sms);
-        case 64: return launch_linear<64, 8, 2, 4>(*d, stream, sms);
+        case 256: return launch_linear<256, 4, 1, 4>(*d, stream, sms, tc.multi_block);
+        case 128: return launch_linear<128, 6, 2, 3>(*d, stream, sms, tc.multi_block);
+        case 64: return launch_linear<64, 8, 2, 4>(*d, stream, sms, tc.multi_block);
         default: return B200_ERR_PARAM;
     }
 }

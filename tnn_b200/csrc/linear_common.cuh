@@ -386,7 +386,7 @@ struct WarpEpilogue {
 
 // CTA-pair kernel (linear_pair.cu).  BN in {64, 128, 192, 256}.
 template <int BN>
-int launch_linear_pair(const B200LinearDesc& d, cudaStream_t stream, int sm_count);
+int launch_linear_pair(const B200LinearDesc& d, cudaStream_t stream, int sm_count, bool multi_block);
 int device_sm_count();   // SMs of the current device, <= 0 if it is not an sm_100 GPU
 // Argument checks of b200_linear_fwd (pointers, alignment, leading dimensions, epilogue consistency).
 int validate_linear_desc(const B200LinearDesc* d);

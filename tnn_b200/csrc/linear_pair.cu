@@ -349,20 +349,20 @@ int max_active_pairs(int bn) {
 template <int BN, bool RES> constexpr int pair_ksub() { return BN == 64 || (BN == 128 && !RES) ? 2 : 1; }
 
 template <int BN>
-int launch_linear_pair(const B200LinearDesc& d, cudaStream_t stream, int sm_count) {
+int launch_linear_pair(const B200LinearDesc& d, cudaStream_t stream, int sm_count, bool multi_block) {
     // The TMA residual path needs 16-byte aligned residual rows (checked by the caller) and a half-precision residual.
     const bool res = d.epilogue == B200_EPI_BIAS_RESIDUAL;
     if (wants_fold(d)) return res ? launch_pair<BN, true, true, 1>(d, stream, sm_count) : launch_pair<BN, false, true, 1>(d, stream, sm_count);
-    if (d.K % BK == 0)
+    if (multi_block)
         return res ? launch_pair<BN, true, false, pair_ksub<BN, true>()>(d, stream, sm_count)
                    : launch_pair<BN, false, false, pair_ksub<BN, false>()>(d, stream, sm_count);
     return res ? launch_pair<BN, true, false, 1>(d, stream, sm_count) : launch_pair<BN, false, false, 1>(d, stream, sm_count);
 }
 
-template int launch_linear_pair<256>(const B200LinearDesc&, cudaStream_t, int);
-template int launch_linear_pair<192>(const B200LinearDesc&, cudaStream_t, int);
-template int launch_linear_pair<128>(const B200LinearDesc&, cudaStream_t, int);
-template int launch_linear_pair<64>(const B200LinearDesc&, cudaStream_t, int);
+template int launch_linear_pair<256>(const B200LinearDesc&, cudaStream_t, int, bool);
+template int launch_linear_pair<192>(const B200LinearDesc&, cudaStream_t, int, bool);
+template int launch_linear_pair<128>(const B200LinearDesc&, cudaStream_t, int, bool);
+template int launch_linear_pair<64>(const B200LinearDesc&, cudaStream_t, int, bool);
 
 }  // namespace lin
 }  // namespace b200
