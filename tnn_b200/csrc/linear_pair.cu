@@ -272,7 +272,6 @@ int launch_pair(const B200LinearDesc& d, cudaStream_t stream, int sm_count) {
     p.ln_eps = d.ln_eps;
     p.k_slots = (p.K + 31) / 32;
     p.n_slots = (p.N + 31) / 32;
-    p.x_rows = 128;
 
     static PerDeviceOnce attr_once;
     int dev = 0;

@@ -115,10 +115,6 @@ template <int N>
 __device__ __forceinline__ void tma_store_wait_read() {
     asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
-template <int N>
-__device__ __forceinline__ void tma_store_wait_all() {
-    asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
-}
 
 // ---------------------------------------------------------------- TMEM
 // Executed by one full warp.  `ncols` is a power of two in [32, 512].  The base address lands in *dst_smem.
