@@ -572,7 +572,9 @@ attention_pingpong_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, c
         Item it;
         // Heads vary fastest, then the query blocks of a sequence: with the query blocks fastest and an even number of them,
         // a grid of 148 dealt every second CTA nothing but last blocks, which for S = 384 (a last block of 128 queries
-        // instead of 256) left half of the CTAs with half of the work: 64 x 384 tokens, 16 heads: 110.9 us, now 101.7.
+        // instead of 256) left half of the CTAs with half of the work: 64 x 384 tokens, 16 heads: 110.9 us, now 101.7.  With
+        // three of them it is the other way round where the last one is short (16 x 520 64.4 query blocks first, 66.8 heads
+        // first; 8 x 640 36.0, 36.8) and the same way where it is not (16 x 768 81.8, 80.3).
         it.head = id % p.heads;
         const int rest = id / p.heads;
         const int qb = rest % p.n_qb;
@@ -1269,8 +1271,9 @@ int launch_pingpong(AttnParams& p, int dtype, long long S, int heads, long long 
         const dim3 block(PPCfg<PP_NWG, 2>::THREADS);
         constexpr size_t smem = PPCfg<PP_NWG, 2>::SMEM;
         // Issuers as one lane up to six key tiles, as a whole warp beyond, us per launch with 16 or 12 heads, whole warp ->
-        // one lane: 64 x 384 101.7 -> 93.8, 16 x 512 40.0 -> 39.4, 32 x 256 21.7 -> 20.7, 8 x 640 (100 .. 640 valid) 27.9 ->
-        // 26.0;  16 x 1024 116.1 -> 120.4, of 200 .. 1024 valid 96.8 -> 98.9.
+        // one lane: 64 x 384 101.7 -> 93.8, 16 x 512 41.4 -> 40.9, 32 x 256 21.7 -> 20.7, 8 x 640 37.2 -> 36.8 and of 100 .. 640
+        // valid 30.3 -> 29.2, 16 x 700 57.3 -> 57.5 and of 100 .. 700 valid 58.9 -> 57.0;  at 768 full and padded batches part:
+        // 16 x 768 78.6 -> 80.3, of 100 .. 768 valid 63.5 -> 62.2;  16 x 1024 116.1 -> 120.4, of 200 .. 1024 valid 96.8 -> 98.9.
         const bool one = S <= 6 * TK;
         auto kernel = dtype == B200_F16
                           ? (one ? attention_pingpong_persistent_kernel<B200_F16, PP_NWG, true>

@@ -12,10 +12,10 @@
 //                                   issuer fills b^1.
 // Used where a launch has few tiles; what bounds it there is one tile's serial chain of stages.  The hand-shake of a stage
 // (wait, fence, UMMAs, commit) takes ~270 clocks whatever it holds, measured with the loads left out and a single UMMA per
-// k-block (5.1 of the 7 us that 36 more k-blocks take on a 128 x 64 tile); the UMMAs of a k-block take 50-120.  Hence several
-// k-blocks per stage, each operand fetched by one 3-D TMA box: 3072 -> 768 at 41 rows on 64 x 32 tiles 10.2 us with one
-// k-block per stage, 7.5 / 6.7 / 6.3 with two / three / four, 150 clocks per k-block, which is what the SM's read port from
-// L2 needs for the tile's 96 rows of operands.
+// k-block (5.1 of the 7 us that 36 more k-blocks take on a 128 x 64 tile).  Hence several k-blocks per stage, each operand
+// fetched by one 3-D TMA box: 3072 -> 768 at 41 rows on 64 x 32 tiles 10.2 us with one k-block per stage, 7.5 / 6.7 / 6.3 with
+// two / three / four.  A k-block then takes 155-165 clocks of 1965 MHz (slope from 3072 to 6144 deep), of which its loads alone,
+// with the UMMAs left out, would take 101-121 (24 and 144 CTAs): it is still the chain that binds, not the way from L2.
 // Algorithmic work per launch: 2*M*N*K flop; HBM traffic at least (M*K + N*K + M*N (+ M*N residual)) elements.
 #include "linear_common.cuh"
 
@@ -429,9 +429,9 @@ extern "C" int b200_linear_fwd(const B200LinearDesc* d, b200_stream_t stream_) {
     }
     if (tc.tm == 64) {
         if (tc.bn == 64) return launch_linear_t<64, 64, 4, 3, false>(*d, stream, sms);
-        // Up to 48 rows fetch only the rows that exist, rounded up to the swizzle's eight: rows beyond M cross the SM's read
-        // port from L2 as zeros.  us per launch at 16 rows: 768 -> 2304 3.8 -> 3.2, 768 -> 3072 4.6 -> 3.5; at 41 rows 768 -> 3072
-        // 3.95 -> 3.75; at 56 rows and more there is nothing left to gain.
+        // Up to 48 rows fetch only the rows that exist, rounded up to the swizzle's eight: rows beyond M are written to shared
+        // memory as zeros at the cost of loaded ones.  us per launch at 16 rows: 768 -> 2304 3.8 -> 3.2, 768 -> 3072 4.6 -> 3.5;
+        // at 41 rows 768 -> 3072 3.95 -> 3.75; at 56 rows and more there is nothing left to gain.
         return d->M <= 48 ? launch_linear_t<64, 32, 4, 4, false, true>(*d, stream, sms)
                           : launch_linear_t<64, 32, 4, 4, false>(*d, stream, sms);
     }
