@@ -80,8 +80,8 @@ def test_linear_epilogues(cuda_device, dt, epi):
 @pytest.mark.parametrize("dt", ["f16", "bf16"])
 @pytest.mark.parametrize("M,N,K", [
     (1, 8, 64), (8, 776, 320), (41, 768, 768), (48, 136, 1088), (49, 136, 1088),   # 64 x 32 tiles, up to 48 rows: short x boxes
-    (65, 776, 320), (128, 2304, 768),
-    (128, 3072, 832), (200, 2312, 64),                                  # 64 x 64
+    (65, 776, 320), (128, 2304, 768),                                   # (K = 64 and, beyond 64 x 32 tiles, K < 512: one block per stage)
+    (128, 3072, 832), (200, 2312, 64),                                  # 64 x 64, 128 x 64
     (300, 3080, 128),                                                   # 128 x 64
     (520, 3000, 192),                                                   # 128 x 128 (pair tiles with a residual)
     (41, 768, 776),                                                     # K not in whole k-blocks: one block per stage
